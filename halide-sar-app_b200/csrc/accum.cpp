@@ -62,7 +62,7 @@ AccumLayout accum_layout(const sarbp_job &j, int tile_x, int tile_y, int C) {
     L.job = o;     o = a256(o + sizeof(DevJob));
     L.items = o;   o = a256(o + ntiles * sizeof(WorkItem));
     L.rows = o;    o = a256(o + (size_t)C * sizeof(RowItem));
-    L.cnt = o;     o = a256(o + sizeof(int));
+    L.cnt = o;     o = a256(o + kBpCounterBytes);
     L.filt = o;    o = a256(o + S * sizeof(float));
     L.wS = o;      o = a256(o + S * sizeof(float));
     L.wP = o;      o = a256(o + P * sizeof(float));
@@ -212,12 +212,13 @@ int sarbp_accum::add(int q0, int n, const float *phs_rows, cudaEvent_t rc_done) 
                                 lay.work_rows, s);
     if (e == cudaSuccess && rc_done) e = cudaEventRecord(rc_done, s);
     if (e == cudaSuccess) e = launch_tile_records(d_job(), items, ntiles, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, sizeof(int), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, kBpCounterBytes, s);
     if (e != cudaSuccess) return cuda_fail(e, "pulse-chunked job: chunk launches");
     BpLaunch Lc = L;
     const int occ = bp_max_active_blocks(Lc);
     if (occ < 1) return fail(SARBP_ERR_CUDA, "backprojection kernel does not fit on an SM");
     Lc.grid = (int)std::min<long long>((long long)occ * ctx->dev.num_sms, (long long)ntiles);
+    Lc.deal.how = kDealItems;  // one chunk's pulses in every tile
     e = launch_backproject(Lc, d_job(), items, ntiles, cnt, s);
     if (e != cudaSuccess) return cuda_fail(e, "pulse-chunked job: backprojection launch");
     ctx->dev.launches += 5;

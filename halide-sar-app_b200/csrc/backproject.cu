@@ -31,13 +31,18 @@
 // parts outside the profile are filled with the clamped edge pair), both
 // completing on mbarriers with bounded waits.  Hand-over uses named
 // barriers: FULL[b] producer -> consumers, EMPTY[b] consumers -> producer;
-// each instance gets one arrival set from each side, and the producer
-// drains the last two EMPTY instances of every tile.
+// each instance gets one arrival set from each side.  The chunks of a CTA's
+// items form one sequence (chunk g in half g & 1), so the producer stages the
+// next item's first chunks while the consumers still work on the last ones of
+// the current item; it drains the last EMPTY instance at the end.
 //
 // Work list: items are (job, tile, pulse part); with `persistent` the grid
-// is the number of resident CTAs and each CTA pulls items (ordered longest
-// first by the host) from an atomic counter, so uneven jobs of a batch share
-// one launch.  A job with too few tiles to fill the resident CTAs has each
+// is the number of resident CTAs, CTA i starts with item i, and its producer
+// claims further items (ordered longest first by the host) from an atomic
+// counter as it finishes staging the current one, so uneven jobs of a batch
+// share one launch.  Towards the end of the list the SMs take even shares (see
+// Claims::next).
+// A job with too few tiles to fill the resident CTAs has each
 // tile split into nsplit items over consecutive pulse ranges; each stores
 // its sums into its own slice of the job's parts buffer (plain stores, no
 // atomics), and the combine kernel adds the slices in a fixed order.
@@ -58,7 +63,6 @@ constexpr float kMagic = 12582912.0f;             // 1.5 * 2^23
 constexpr uint32_t kMagicBits = 0x4B400000u;
 constexpr uint32_t kMagicOff = kMagicBits << 4;   // (mod 2^32) byte offset of index 0
 constexpr int kConsumers = 256;                   // consumer threads (8 warps)
-constexpr int kConsumerWarps = kConsumers / 32;
 constexpr int kThreads = kConsumers + 32;         // plus one producer warp
 constexpr int kBarFull0 = 1;                      // named barriers 1, 2: chunk staged
 constexpr int kBarEmpty0 = 3;                     // named barriers 3, 4: chunk consumed
@@ -74,6 +78,15 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
 }
 __device__ __forceinline__ double warp_max(double v) {
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+__device__ __forceinline__ int4 lds_int4(const int4 *p) {
+    int4 v;
+    asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(smem_u32(p))
+                 : "memory");
     return v;
 }
 
@@ -126,7 +139,7 @@ __device__ __forceinline__ void bulk_copy(void *dst, const void *src, uint32_t b
 // instruction, the same rounding as two scalar operations), so every
 // per-pixel FP32 step up to the range bin costs half an issue slot; the
 // window loads, the interpolation and the sine/cosine stay per pixel.  Each
-// record is staged as four float4 of broadcast pairs (see stage_chunk).
+// record is staged as four float4 of broadcast pairs (see stage_windows).
 // The images are the same bit for bit as with scalar arithmetic.
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
@@ -275,6 +288,28 @@ __device__ __forceinline__ void accumulate_mode(int mode, bool planar, int nc, c
 #undef SARBP_ACC
 }
 
+// What the consumers need of an item besides its chunks, written by the
+// producer ahead of the item's first chunk: the consumers' item set-up and
+// epilogue then wait for one level of global loads (positions; final phases
+// or sums) instead of a chain of four (item, job, tile, values) and a read
+// and a write in turn for each pixel.  1024^2 pixels, 200-pulse chunks added
+// to a partial image: 282 us a chunk with the chain, 171 without.
+struct __align__(16) ItemCtx {
+    double rc[3], uh[3], vh[3];
+    const double *r, *u, *v;
+    const float2 *fin;  // [nv][nu] final phases
+    float2 *sums;       // kItemAcc: partial image; kItemPart: the part's slice
+    double2 *out;
+    JobScalars *sc;
+    float w0[3], kcf;
+    float ilk;  // range bins per radian of Delta
+    int nu, nv, tx0, ty0, flags;
+};
+constexpr int kItemTransposed = 1, kItemAcc = 2, kItemPart = 4, kItemMax = 8, kItemTooWide = 16;
+// An item's slot is rewritten four items later, when the consumers have long
+// passed its epilogue (the producer is at most two chunks ahead).
+constexpr int kCtxSlots = 4;
+
 // Shared memory of the tile kernel.
 struct TileSmem {
     float4 *stage;       // [2][stage_cap] (m, d) windows
@@ -282,13 +317,20 @@ struct TileSmem {
     float4 *rec2;        // [2][4 cmax] records as broadcast pairs (see accumulate)
     uint64_t *mbar_rec;  // [2]
     uint64_t *mbar_win;  // [2]
-    double *sred;        // [kConsumerWarps]
-    int *s_item, *s_mode;
+    int4 *s_chunk;       // [2] what each half holds (see below)
+    ItemCtx *ctx;        // [kCtxSlots] constants of the items in flight
 };
 
 struct TileShape {
     int K, W, C, nchunks;
 };
+
+// What the producer tells the consumers about a staged chunk, one int4 a half:
+// x = context slot of its item (-1: no more), y = pulses in the chunk, z = window stride (bytes),
+// w = series mode | flags below.  The consumers read it from shared memory at
+// every chunk rather than carry it through the pulse loop, whose registers
+// are what limits the kernel at 3 CTAs per SM.
+constexpr int kChunkPlanar = 4, kChunkWide = 8, kChunkFirst = 16, kChunkLast = 32;
 
 // Chunking of an item's np pulses: C pulses per chunk (the windows of a
 // chunk fill at most one staging half), nchunks chunks.
@@ -304,13 +346,10 @@ __device__ __forceinline__ TileShape tile_shape(const TileInfo &t, int np, int s
     return s;
 }
 
-// Producer warp, one chunk into half b: records, then windows.
-__device__ __forceinline__ bool stage_chunk(const DevJob &jb, int tile, int lane, int p0, int nc, int b,
-                                            const TileShape &sh, int stage_cap, int cmax,
-                                            const TileSmem &sm, uint32_t (&uses)[4]) {
-    const int N = jb.N, W = sh.W;
+// Producer warp, one chunk into half b: the copy of its records ...
+__device__ __forceinline__ void stage_records(const DevJob &jb, int tile, int lane, int p0, int nc, int b,
+                                              const TileSmem &sm) {
     PulseRec *rec = sm.raw;
-    float4 *win = sm.stage + b * stage_cap;
     // prior generic-proxy reads of these buffers come before the async writes
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (lane == 0) {
@@ -318,12 +357,21 @@ __device__ __forceinline__ bool stage_chunk(const DevJob &jb, int tile, int lane
         bulk_copy(rec, jb.recs + (size_t)tile * jb.P + p0, (uint32_t)(nc * (int)sizeof(PulseRec)),
                   &sm.mbar_rec[b]);
     }
+}
+
+// ... then, once they are there, its windows.
+__device__ __forceinline__ bool stage_windows(const DevJob &jb, int lane, int p0, int nc, int b,
+                                              const TileShape &sh, int stage_cap, int cmax,
+                                              const TileSmem &sm, uint32_t (&uses)[4], int &mode) {
+    const int N = jb.N, W = sh.W;
+    PulseRec *rec = sm.raw;
+    float4 *win = sm.stage + b * stage_cap;
     bool ok = mbar_wait(&sm.mbar_rec[b], uses[b] & 1u);
     uses[b]++;
     // window copies: bins [base, base + W) of row p; the in-profile part
     // [max(base, 0), min(base + W, N)) comes from the pairs row
     uint32_t bytes = 0;
-    int mode = 0;
+    mode = 0;
     for (int i = lane; i < nc; i += 32) {
         const int bits = __float_as_int(rec[i].b.w);
         const int base = bits >> 3, order = bits & 7;
@@ -351,10 +399,7 @@ __device__ __forceinline__ bool stage_chunk(const DevJob &jb, int tile, int lane
         const float e2 = mode == 1 ? ee + ee : ee;
         r2[4 * i + 3] = mode == 3 ? make_float4(q.z, 0.0f, de, de) : make_float4(e2, e2, de, de);
     }
-    if (lane == 0) {
-        sm.s_mode[b] = mode;
-        mbar_expect(&sm.mbar_win[b], bytes);  // the arrival of this phase
-    }
+    if (lane == 0) mbar_expect(&sm.mbar_win[b], bytes);  // the arrival of this phase
     __syncwarp();
     for (int i = lane; i < nc; i += 32) {
         const int bits = __float_as_int(rec[i].b.w);
@@ -376,200 +421,288 @@ __device__ __forceinline__ bool stage_chunk(const DevJob &jb, int tile, int lane
     return ok;
 }
 
+// Launch counters, zero before the launch: [0] items claimed beyond the first
+// of each CTA, [1] SMs that run CTAs of the launch, [2] CTAs started, then
+// from word 4 what the CTAs of each SM took: items, one byte per SM
+// (kDealItems), or pulses, one word per SM (kDealPulses).
+struct Claims {
+    int *ctr;
+    int nitems, grid;
+    BpDeal deal;
+    uint32_t sm;
+
+    // adds an item of `pulses` to the SM's account; what it held before
+    __device__ __forceinline__ long long account(int pulses) {
+        if (deal.how == kDealPulses) return atomicAdd(&ctr[4 + sm % (uint32_t)kBpDealSms], pulses);
+        const uint32_t at = sm % (uint32_t)(kBpCounterBytes - 16), shift = (at & 3u) * 8;
+        return ((uint32_t)atomicAdd(&ctr[4 + (at >> 2)], 1 << shift) >> shift) & 255u;
+    }
+
+    // the CTA's first item, blockIdx.x
+    __device__ __forceinline__ void start(int pulses) {
+        if (deal.how == kDealNone) return;
+        asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+        if (account(pulses) == 0) atomicAdd(&ctr[1], 1);
+        __threadfence();  // [1] is complete once [2] says that all CTAs have started
+        atomicAdd(&ctr[2], 1);
+    }
+
+    // The CTA's next item, or nitems when it has none.  The CTAs of an SM do
+    // not advance alike (the warp schedulers favour the oldest: of 2048^2
+    // pixels' 4096 tiles the three CTAs of an SM take 14, 9 and 5), while the
+    // SMs do.  Left to themselves the first SMs to finish a round of equal
+    // items take one for each of their CTAs (of 736 tiles on 148 SMs up to
+    // six where five suffice), and in an uneven list the slowest CTA of an SM
+    // is left with a long item at the end.  So from item deal.zone on, an SM
+    // that has taken its share deal.total / SMs takes no more.  While items
+    // remain some SM is short of its share, so all are taken; the rule waits
+    // until every CTA has started.  736 tiles x 777 pulses: 532-620 us before,
+    // 489 now; 4096 tiles x 1999: 5.77 -> 5.54 ms; 6 jobs of 256^2 and 512^2
+    // replayed: 457 -> 419 us (nearly all of it this rule).
+    __device__ __forceinline__ int next() {
+        if (deal.how != kDealNone) {
+            const volatile int *v = ctr;
+            const int at = grid + v[0], started = v[2], sms = v[1];
+            if (at >= deal.zone && started == grid) {
+                const long long took = deal.how == kDealPulses
+                    ? (long long)v[4 + sm % (uint32_t)kBpDealSms]
+                    : (long long)reinterpret_cast<const volatile unsigned char *>(
+                          ctr + 4)[sm % (uint32_t)(kBpCounterBytes - 16)];
+                if (took * sms >= deal.total) return nitems;
+            }
+        }
+        return min(nitems, grid + atomicAdd(ctr, 1));
+    }
+};
+
+// An item's constants for the consumers.
+__device__ __forceinline__ void fill_ctx(ItemCtx &c, const DevJob &jb, const WorkItem &wi, int flags) {
+    const TileInfo &t = jb.tiles[wi.tile];
+    const double k_c = jb.sc->k_c;
+    for (int d = 0; d < 3; ++d) {
+        c.rc[d] = t.rc[d];
+        c.uh[d] = jb.uh[d];
+        c.vh[d] = jb.vh[d];
+        c.w0[d] = t.w0[d];
+    }
+    c.r = jb.r;
+    c.u = jb.u;
+    c.v = jb.v;
+    c.fin = jb.fin;
+    c.out = jb.out;
+    c.sc = jb.sc;
+    c.sums = jb.nsplit > 1 ? jb.parts + (long long)wi.part * ((long long)jb.nu * jb.nv) : jb.acc;
+    c.kcf = (float)k_c;
+    c.ilk = (float)(jb.inv_lsr / k_c);
+    c.nu = jb.nu;
+    c.nv = jb.nv;
+    c.tx0 = (wi.tile % jb.tiles_x) * jb.tile_x;
+    c.ty0 = (wi.tile / jb.tiles_x) * jb.tile_y;
+    // only the u8 image uses max|z|
+    c.flags = flags | (t.transposed ? kItemTransposed : 0) |
+              (jb.nsplit > 1 ? kItemPart : jb.acc ? kItemAcc : jb.out_u8 ? kItemMax : 0);
+}
+
 // Producer warp: the same barrier sequence as the consumers.
 __device__ __forceinline__ void producer_loop(const DevJob *__restrict__ jobs,
                                               const WorkItem *__restrict__ items, int nitems,
-                                              int stage_cap, int cmax, int persistent, const TileSmem &sm) {
+                                              int *__restrict__ counter, int stage_cap, int cmax,
+                                              int persistent, const BpDeal &deal, const TileSmem &sm) {
     const int lane = threadIdx.x & 31;
     // completed phases of each mbarrier: records [0..1], windows [2..3]
     uint32_t uses[4] = {0u, 0u, 0u, 0u};
+    Claims claims{counter, nitems, (int)gridDim.x, deal, 0};
     int item = blockIdx.x;
-    for (;;) {
-        if (persistent) {
-            __syncthreads();  // s_item written
-            item = *sm.s_item;
+    int g = 0;  // chunks staged so far
+    for (int n = 0;; ++n) {
+        // Claim late, once the consumers are done with chunk g-2: an item is
+        // not held back by a CTA that still has two chunks to go
+        if (g >= 2) bar_sync(kBarEmpty0 + (g & 1));
+        if (n > 0) {
+            int nxt = nitems;
+            if (persistent && lane == 0) nxt = claims.next();
+            item = __shfl_sync(0xffffffffu, nxt, 0);
         }
-        if (item >= nitems) break;
-        const WorkItem wi = items[item];
+        const bool more = item < nitems;
+        const WorkItem wi = more ? items[item] : WorkItem{0, 0, 0};
         const DevJob &jb = jobs[wi.job];
-        int pb, pe;  // the item's pulses
-        part_range(jb.P, jb.nsplit, wi.part, pb, pe);
-        const TileShape sh = tile_shape(jb.tiles[wi.tile], pe - pb, stage_cap, cmax);
+        int pb = 0, pe = 0;  // the item's pulses
+        TileShape sh{0, 1, 1, 0};
+        int flags = 0;
+        if (more) {
+            part_range(jb.P, jb.nsplit, wi.part, pb, pe);
+            const TileInfo &ti = jb.tiles[wi.tile];
+            sh = tile_shape(ti, pe - pb, stage_cap, cmax);
+            flags = (ti.planar ? kChunkPlanar : 0) | (ti.wide ? kChunkWide : 0);
+            if (persistent && lane == 0) {
+                if (n == 0) claims.start(pe - pb);
+                else if (deal.how != kDealNone) claims.account(pe - pb);
+            }
+        }
         bool ok = true;
-        for (int c = 0; c < sh.nchunks; ++c) {
-            const int b = c & 1;
-            if (c >= 2) bar_sync(kBarEmpty0 + b);  // consumers are done with chunk c-2
-            const int p0 = pb + c * sh.C;
-            ok = stage_chunk(jb, wi.tile, lane, p0, min(sh.C, pe - p0), b, sh, stage_cap, cmax, sm, uses) &&
-                 ok;
+        // an item without chunks (tile too wide) and the end take one empty turn
+        const int turns = max(sh.nchunks, 1);
+        for (int c = 0; c < turns; ++c, ++g) {
+            const int b = g & 1;
+            if (c > 0 && g >= 2) bar_sync(kBarEmpty0 + b);  // consumers are done with chunk g-2
+            int nc = 0, mode = 0;
+            if (c < sh.nchunks) {
+                const int p0 = pb + c * sh.C;
+                nc = min(sh.C, pe - p0);
+                stage_records(jb, wi.tile, lane, p0, nc, b, sm);
+            }
+            if (c == 0 && more && lane == 0)
+                fill_ctx(sm.ctx[n & (kCtxSlots - 1)], jb, wi, sh.C < 1 ? kItemTooWide : 0);
+            if (c < sh.nchunks)
+                ok = stage_windows(jb, lane, pb + c * sh.C, nc, b, sh, stage_cap, cmax, sm, uses, mode) && ok;
+            if (lane == 0)
+                sm.s_chunk[b] = make_int4(more ? n & (kCtxSlots - 1) : -1, nc, sh.W * 16,
+                                          mode | flags | (c == 0 ? kChunkFirst : 0) |
+                                              (c == turns - 1 ? kChunkLast : 0));
+            __syncwarp();
             bar_arrive(kBarFull0 + b);
         }
-        for (int c = sh.nchunks > 2 ? sh.nchunks - 2 : 0; c < sh.nchunks; ++c) bar_sync(kBarEmpty0 + (c & 1));
+        if (!more) break;
         if (!ok && lane == 0) atomicOr(&jb.sc->status, kStatusTimeout);
-        __syncthreads();  // epilogue partials
-        if (!persistent) break;
     }
+    // the consumers' arrival on the last chunk before the end's empty turn
+    if (g >= 2) bar_sync(kBarEmpty0 + (g & 1));
 }
 
 template <int TX, int TY, bool PRE>
-__device__ __forceinline__ void consumer_loop(const DevJob *__restrict__ jobs,
-                                              const WorkItem *__restrict__ items, int nitems,
-                                              int *__restrict__ counter, int stage_cap, int cmax,
-                                              int persistent, const TileSmem &sm) {
+__device__ __forceinline__ void consumer_loop(int stage_cap, int cmax, const TileSmem &sm) {
     constexpr int PPT = TX * TY / kConsumers;
     constexpr int ROWS = kConsumers / TX;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int lx = tid % TX, ly = tid / TX;
+    const int tid = threadIdx.x;
     // pixel k of this thread: lanes run along x, or along y on transposed
     // tiles (square tiles whose range bins step faster along x than along y,
     // so that neighbouring lanes read neighbouring or equal window entries)
-    auto pixel_of = [&](bool tr, int tx0, int ty0, int k, int &ix, int &iy) {
-        if (TX == TY && tr) {
-            ix = tx0 + ly + k * ROWS;
-            iy = ty0 + lx;
+    auto pixel_of = [&](const ItemCtx &it, int k, int &ix, int &iy) {
+        const int lx = tid % TX, ly = tid / TX;
+        if (TX == TY && (it.flags & kItemTransposed)) {
+            ix = it.tx0 + ly + k * ROWS;
+            iy = it.ty0 + lx;
         } else {
-            ix = tx0 + lx;
-            iy = ty0 + ly + k * ROWS;
+            ix = it.tx0 + lx;
+            iy = it.ty0 + ly + k * ROWS;
         }
     };
     const uint32_t stage_base = smem_u32(sm.stage) - kMagicOff;
-    int item = blockIdx.x;
-    for (;;) {
-        if (persistent) {
-            if (tid == 0) *sm.s_item = atomicAdd(counter, 1);
-            __syncthreads();
-            item = *sm.s_item;
-        }
-        if (item >= nitems) break;
-        const WorkItem wi = items[item];
-        const DevJob &jb = jobs[wi.job];
-        const int nu = jb.nu, nv = jb.nv, P = jb.P;
-        const int tx0 = (wi.tile % jb.tiles_x) * TX;
-        const int ty0 = (wi.tile / jb.tiles_x) * TY;
-        const TileInfo ti = jb.tiles[wi.tile];
-        int pb, pe;  // the item's pulses
-        part_range(P, jb.nsplit, wi.part, pb, pe);
-        const TileShape sh = tile_shape(ti, pe - pb, stage_cap, cmax);
-        const double k_c = jb.sc->k_c;
-        const float kcf = (float)k_c;
-
-        // ---- pixel offsets from the tile centre, in radians ----
-        float dx[PPT], dy[PPT], dz[PPT], nd2[PPT], s0[PPT];
+    constexpr int NP = PPT / 2;
+    // pixel pairs (2j, 2j + 1) for the f32x2 arithmetic
+    float2 dxp[NP], dyp[NP], dzp[NP], nd2p[NP], s0p[NP], arp[NP], aip[NP];
+    float ilk = 0.0f;
+    for (int b = 0;; b ^= 1) {
+        bar_sync(kBarFull0 + b);
+        const int4 ch = lds_int4(&sm.s_chunk[b]);
+        if (ch.x < 0) break;
+        if (ch.w & kChunkFirst) {
+            // ---- pixel offsets from the tile centre, in radians ----
+            const ItemCtx &it = sm.ctx[ch.x];
+            ilk = it.ilk;
+            double x[PPT], y[PPT], z[PPT];
+            bool in[PPT];
+            // all positions are loaded before the first is used (pixels
+            // outside the image read the edge's and are dropped below)
 #pragma unroll
-        for (int k = 0; k < PPT; ++k) {
-            int ix, iy;
-            pixel_of(ti.transposed != 0, tx0, ty0, k, ix, iy);
-            dx[k] = dy[k] = dz[k] = nd2[k] = s0[k] = 0.0f;
-            if (ix < nu && iy < nv) {
-                double x, y, z;
-                if (jb.r) {
-                    const long long npix = (long long)nu * nv;
-                    const long long pix = (long long)iy * nu + ix;
-                    x = jb.r[pix];
-                    y = jb.r[npix + pix];
-                    z = jb.r[2 * npix + pix];
+            for (int k = 0; k < PPT; ++k) {
+                int ix, iy;
+                pixel_of(it, k, ix, iy);
+                in[k] = ix < it.nu && iy < it.nv;
+                ix = min(ix, it.nu - 1);
+                iy = min(iy, it.nv - 1);
+                if (it.r) {
+                    const long long npix = (long long)it.nu * it.nv;
+                    const long long pix = (long long)iy * it.nu + ix;
+                    x[k] = it.r[pix];
+                    y[k] = it.r[npix + pix];
+                    z[k] = it.r[2 * npix + pix];
                 } else {
                     // img_plane.cpp:92-102: (0 + u_hat*u) + v_hat*v
-                    const double uu = jb.u[ix], vv = jb.v[iy];
-                    x = __dadd_rn(__dmul_rn(jb.uh[0], uu), __dmul_rn(jb.vh[0], vv));
-                    y = __dadd_rn(__dmul_rn(jb.uh[1], uu), __dmul_rn(jb.vh[1], vv));
-                    z = __dadd_rn(__dmul_rn(jb.uh[2], uu), __dmul_rn(jb.vh[2], vv));
-                }
-                if (isfinite(x) && isfinite(y) && isfinite(z)) {
-                    // the same f32 offsets the tile set-up measured rho on
-                    dx[k] = kcf * (float)(x - ti.rc[0]);
-                    dy[k] = kcf * (float)(y - ti.rc[1]);
-                    dz[k] = kcf * (float)(z - ti.rc[2]);
-                    nd2[k] = -fmaf(dx[k], dx[k], fmaf(dy[k], dy[k], dz[k] * dz[k]));
-                    s0[k] = fmaf(ti.w0[2], dz[k], fmaf(ti.w0[1], dy[k], ti.w0[0] * dx[k]));
+                    const double uu = it.u[ix], vv = it.v[iy];
+                    x[k] = __dadd_rn(__dmul_rn(it.uh[0], uu), __dmul_rn(it.vh[0], vv));
+                    y[k] = __dadd_rn(__dmul_rn(it.uh[1], uu), __dmul_rn(it.vh[1], vv));
+                    z[k] = __dadd_rn(__dmul_rn(it.uh[2], uu), __dmul_rn(it.vh[2], vv));
                 }
             }
-        }
-        // pixel pairs (2j, 2j + 1) for the f32x2 arithmetic
-        constexpr int NP = PPT / 2;
-        float2 dxp[NP], dyp[NP], dzp[NP], nd2p[NP], s0p[NP], arp[NP], aip[NP];
+            float dx[PPT], dy[PPT], dz[PPT], nd2[PPT], s0[PPT];
 #pragma unroll
-        for (int j = 0; j < NP; ++j) {
-            dxp[j] = make_float2(dx[2 * j], dx[2 * j + 1]);
-            dyp[j] = make_float2(dy[2 * j], dy[2 * j + 1]);
-            dzp[j] = make_float2(dz[2 * j], dz[2 * j + 1]);
-            nd2p[j] = make_float2(nd2[2 * j], nd2[2 * j + 1]);
-            s0p[j] = make_float2(s0[2 * j], s0[2 * j + 1]);
-            arp[j] = aip[j] = make_float2(0.0f, 0.0f);
-        }
-        if (sh.C < 1) {
-            if (tid == 0) atomicOr(&jb.sc->status, kStatusTileTooWide);
-        } else {
-            const float ilk = (float)(jb.inv_lsr / k_c);  // range bins per radian of Delta
-            const float2 ILK = make_float2(ilk, ilk);
-            const float2 CL = f2(0.0f, (float)(sh.W - 1) - 0.5f);  // bin-argument clamp (modes 2, 3)
-            const uint32_t pstride = (uint32_t)sh.W * 16u;
-            for (int c = 0; c < sh.nchunks; ++c) {
-                const int b = c & 1;
-                bar_sync(kBarFull0 + b);
-                const int p0 = pb + c * sh.C;
-                const uint32_t poff = stage_base + (uint32_t)(b * stage_cap) * 16u;
-                const int nc = min(sh.C, pe - p0);
-                const float4 *rec2 = sm.rec2 + (size_t)b * 4 * cmax;
-                if (ti.wide)
-                    accumulate_mode<true, NP, PRE>(sm.s_mode[b], ti.planar != 0, nc, rec2, poff, pstride, ILK, CL,
-                                              dxp, dyp, dzp, nd2p, s0p, arp, aip);
-                else
-                    accumulate_mode<false, NP, PRE>(sm.s_mode[b], ti.planar != 0, nc, rec2, poff, pstride, ILK, CL,
-                                               dxp, dyp, dzp, nd2p, s0p, arp, aip);
-                bar_arrive(kBarEmpty0 + b);
+            for (int k = 0; k < PPT; ++k) {
+                dx[k] = dy[k] = dz[k] = nd2[k] = s0[k] = 0.0f;
+                if (in[k] && isfinite(x[k]) && isfinite(y[k]) && isfinite(z[k])) {
+                    // the same f32 offsets the tile set-up measured rho on
+                    dx[k] = it.kcf * (float)(x[k] - it.rc[0]);
+                    dy[k] = it.kcf * (float)(y[k] - it.rc[1]);
+                    dz[k] = it.kcf * (float)(z[k] - it.rc[2]);
+                    nd2[k] = -fmaf(dx[k], dx[k], fmaf(dy[k], dy[k], dz[k] * dz[k]));
+                    s0[k] = fmaf(it.w0[2], dz[k], fmaf(it.w0[1], dy[k], it.w0[0] * dx[k]));
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < NP; ++j) {
+                dxp[j] = make_float2(dx[2 * j], dx[2 * j + 1]);
+                dyp[j] = make_float2(dy[2 * j], dy[2 * j + 1]);
+                dzp[j] = make_float2(dz[2 * j], dz[2 * j + 1]);
+                nd2p[j] = make_float2(nd2[2 * j], nd2[2 * j + 1]);
+                s0p[j] = make_float2(s0[2 * j], s0[2 * j + 1]);
+                arp[j] = aip[j] = make_float2(0.0f, 0.0f);
             }
         }
+        {
+            const float2 ILK = make_float2(ilk, ilk);
+            const uint32_t pstride = (uint32_t)ch.z;
+            // bin-argument clamp (modes 2, 3): W - 1 - 1/2
+            const float2 CL = f2(0.0f, (float)((int)(pstride >> 4) - 1) - 0.5f);
+            const uint32_t poff = stage_base + (uint32_t)(b * stage_cap) * 16u;
+            const float4 *rec2 = sm.rec2 + (size_t)b * 4 * cmax;
+            if (ch.w & kChunkWide)
+                accumulate_mode<true, NP, PRE>(ch.w & 3, (ch.w & kChunkPlanar) != 0, ch.y, rec2, poff, pstride, ILK,
+                                               CL, dxp, dyp, dzp, nd2p, s0p, arp, aip);
+            else
+                accumulate_mode<false, NP, PRE>(ch.w & 3, (ch.w & kChunkPlanar) != 0, ch.y, rec2, poff, pstride, ILK,
+                                                CL, dxp, dyp, dzp, nd2p, s0p, arp, aip);
+        }
+        const int4 done = lds_int4(&sm.s_chunk[b]);  // again, not through the loop
+        bar_arrive(kBarEmpty0 + b);
+        if (!(done.w & kChunkLast)) continue;
         // ---- final phase, row flip (backprojection.cpp:130-138), max|z|;
         // a pulse part stores its sums into its slice, a pulse chunk adds
-        // them to the partial image instead ----
-        double zmax = 0.0;
-        if (jb.nsplit > 1) {
-            float2 *slice = jb.parts + (long long)wi.part * ((long long)nu * nv);
-#pragma unroll
-            for (int k = 0; k < PPT; ++k) {
-                int ix, iy;
-                pixel_of(ti.transposed != 0, tx0, ty0, k, ix, iy);
-                if (ix < nu && iy < nv)
-                    slice[(long long)iy * nu + ix] = make_float2((k & 1) ? arp[k >> 1].y : arp[k >> 1].x,
-                                                                 (k & 1) ? aip[k >> 1].y : aip[k >> 1].x);
-            }
-        } else if (jb.acc) {
-#pragma unroll
-            for (int k = 0; k < PPT; ++k) {
-                int ix, iy;
-                pixel_of(ti.transposed != 0, tx0, ty0, k, ix, iy);
-                if (ix < nu && iy < nv) {
-                    float2 *a = jb.acc + (long long)iy * nu + ix;
-                    const float2 s = *a;
-                    *a = make_float2(s.x + ((k & 1) ? arp[k >> 1].y : arp[k >> 1].x),
-                                     s.y + ((k & 1) ? aip[k >> 1].y : aip[k >> 1].x));
-                }
-            }
-        } else
+        // them to the partial image instead; loads before the first store ----
+        const ItemCtx &it = sm.ctx[done.x];
+        if ((it.flags & kItemTooWide) && tid == 0) atomicOr(&it.sc->status, kStatusTileTooWide);
+        const bool has_sums = (it.flags & (kItemPart | kItemAcc)) != 0;
+        float2 in[PPT];  // final phases, or the partial image so far
 #pragma unroll
         for (int k = 0; k < PPT; ++k) {
             int ix, iy;
-            pixel_of(ti.transposed != 0, tx0, ty0, k, ix, iy);
-            if (ix < nu && iy < nv) {
-                const float2 f = jb.fin[(long long)iy * nu + ix];
-                const float ark = (k & 1) ? arp[k >> 1].y : arp[k >> 1].x;
-                const float aik = (k & 1) ? aip[k >> 1].y : aip[k >> 1].x;
-                const double zr = (double)fmaf(ark, f.x, -aik * f.y);
-                const double zi = (double)fmaf(ark, f.y, aik * f.x);
-                jb.out[(long long)(nv - 1 - iy) * nu + ix] = make_double2(zr, zi);
-                zmax = fmax(zmax, sqrt(zr * zr + zi * zi));
+            pixel_of(it, k, ix, iy);
+            in[k] = make_float2(0.0f, 0.0f);
+            if (ix < it.nu && iy < it.nv && !(it.flags & kItemPart))
+                in[k] = (has_sums ? it.sums : it.fin)[(long long)iy * it.nu + ix];
+        }
+        double zmax = 0.0;
+#pragma unroll
+        for (int k = 0; k < PPT; ++k) {
+            int ix, iy;
+            pixel_of(it, k, ix, iy);
+            if (ix >= it.nu || iy >= it.nv) continue;
+            const float ark = (k & 1) ? arp[k >> 1].y : arp[k >> 1].x;
+            const float aik = (k & 1) ? aip[k >> 1].y : aip[k >> 1].x;
+            if (it.flags & kItemPart) {
+                it.sums[(long long)iy * it.nu + ix] = make_float2(ark, aik);
+            } else if (it.flags & kItemAcc) {
+                it.sums[(long long)iy * it.nu + ix] = make_float2(in[k].x + ark, in[k].y + aik);
+            } else {
+                const double zr = (double)fmaf(ark, in[k].x, -aik * in[k].y);
+                const double zi = (double)fmaf(ark, in[k].y, aik * in[k].x);
+                it.out[(long long)(it.nv - 1 - iy) * it.nu + ix] = make_double2(zr, zi);
+                if (it.flags & kItemMax) zmax = fmax(zmax, sqrt(zr * zr + zi * zi));
             }
         }
-        zmax = warp_max(zmax);
-        if (lane == 0) sm.sred[warp] = zmax;
-        __syncthreads();
-        if (tid == 0 && !jb.acc && jb.nsplit <= 1) {
-            double m = 0.0;
-            for (int w = 0; w < kConsumerWarps; ++w) m = fmax(m, sm.sred[w]);
-            atomicMax(&jb.sc->maxabs, (unsigned long long)__double_as_longlong(m));
+        if (it.flags & kItemMax) {
+            zmax = warp_max(zmax);
+            if ((tid & 31) == 0) atomicMax(&it.sc->maxabs, (unsigned long long)__double_as_longlong(zmax));
         }
-        if (!persistent) break;
     }
 }
 
@@ -580,11 +713,12 @@ template <int TX, int TY, int MINB>
 __global__ void __launch_bounds__(kThreads, MINB) bp_tile_kernel(const DevJob *__restrict__ jobs,
                                                                  const WorkItem *__restrict__ items,
                                                                  int nitems, int *__restrict__ counter,
-                                                                 int stage_cap, int cmax, int persistent) {
+                                                                 int stage_cap, int cmax, int persistent,
+                                                                 BpDeal deal) {
     static_assert(TX * TY % (2 * kConsumers) == 0, "tile must give each consumer pairs of pixels");
     extern __shared__ float4 smem[];
-    __shared__ double sred[kConsumerWarps];
-    __shared__ int s_item, s_mode[2];
+    __shared__ int4 s_chunk[2];
+    __shared__ ItemCtx s_ctx[kCtxSlots];
     __shared__ uint64_t mbar[4];
     TileSmem sm;
     sm.stage = smem;
@@ -592,9 +726,8 @@ __global__ void __launch_bounds__(kThreads, MINB) bp_tile_kernel(const DevJob *_
     sm.rec2 = smem + 2 * stage_cap + 2 * cmax;
     sm.mbar_rec = mbar;
     sm.mbar_win = mbar + 2;
-    sm.sred = sred;
-    sm.s_item = &s_item;
-    sm.s_mode = s_mode;
+    sm.s_chunk = s_chunk;
+    sm.ctx = s_ctx;
     if (threadIdx.x == kConsumers) {
         for (int i = 0; i < 4; ++i)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[i])) : "memory");
@@ -602,9 +735,9 @@ __global__ void __launch_bounds__(kThreads, MINB) bp_tile_kernel(const DevJob *_
     }
     __syncthreads();
     if (__shfl_sync(0xffffffffu, (int)threadIdx.x, 0) >= kConsumers)
-        producer_loop(jobs, items, nitems, stage_cap, cmax, persistent, sm);
+        producer_loop(jobs, items, nitems, counter, stage_cap, cmax, persistent, deal, sm);
     else
-        consumer_loop<TX, TY, (MINB >= 3)>(jobs, items, nitems, counter, stage_cap, cmax, persistent, sm);
+        consumer_loop<TX, TY, (MINB >= 3)>(stage_cap, cmax, sm);
 }
 
 // ---- naive FP32 kernel: one thread per pixel ----
@@ -713,10 +846,18 @@ cudaError_t launch_backproject(const BpLaunch &L, const DevJob *d_jobs, const Wo
     const size_t smem = bp_smem_bytes(L);
     const int grid = L.persistent ? L.grid : nitems;
     if (grid <= 0) return cudaSuccess;
+    BpDeal deal = L.persistent ? L.deal : BpDeal{kDealNone, 0, 0};
+    if (deal.how == kDealItems) {  // equal items: the last round is dealt out
+        deal.zone = nitems - grid;
+        deal.total = nitems;
+        // an SM's count of items is one byte
+        if (nitems >= 200ll * grid / 3) deal.how = kDealNone;
+    }
 #define X(a, b, m)                                                                                \
     if (L.tile_x == a && L.tile_y == b && L.minb == m) {                                          \
         bp_tile_kernel<a, b, m><<<grid, kThreads, smem, st>>>(d_jobs, d_items, nitems, d_counter, \
-                                                              L.stage_cap, L.cmax, L.persistent); \
+                                                              L.stage_cap, L.cmax, L.persistent, \
+                                                              deal);                              \
         return cudaGetLastError();                                                                \
     }
     SARBP_BP_TILES(X)

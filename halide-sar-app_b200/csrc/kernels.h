@@ -33,6 +33,16 @@ cudaError_t launch_range_compress_large(int logN, const DevJob *d_jobs, const Ro
                                         float2 *work, int work_rows, cudaStream_t st);
 
 // backproject.cu
+// Persistent launches: from item `zone` of the list on, an SM takes another
+// item only while what it took is below total / SMs, counted in items
+// (kDealItems: all equally long; zone and total are set by the launch) or in
+// pulses (kDealPulses).
+enum { kDealNone = 0, kDealItems = 1, kDealPulses = 2 };
+struct BpDeal {
+    int how;
+    int zone;
+    long long total;
+};
 struct BpLaunch {
     int tile_x, tile_y;
     int minb;        // CTAs per SM the kernel's registers are sized for (2 or 3)
@@ -40,12 +50,16 @@ struct BpLaunch {
     int cmax;        // max pulses per chunk
     int persistent;  // 1: grid = resident CTAs pulling items from *counter
     int grid;        // CTAs when persistent
+    BpDeal deal;     // how a persistent launch shares out the end of its list
     int parts;       // requested pulse parts per tile (sarbp_opts::pulse_parts)
 };
 bool bp_tile_supported(int tile_x, int tile_y, int minb);
 size_t bp_smem_bytes(const BpLaunch &L);
 int bp_max_active_blocks(const BpLaunch &L);
 cudaError_t init_backproject_attributes();
+// d_counter: kBpCounterBytes of device memory (kBpDealBytes with kDealPulses),
+// zero before a persistent launch
+constexpr int kBpCounterBytes = 256, kBpDealSms = 252, kBpDealBytes = 16 + 4 * kBpDealSms;
 cudaError_t launch_backproject(const BpLaunch &L, const DevJob *d_jobs, const WorkItem *d_items,
                                int nitems, int *d_counter, cudaStream_t st);
 cudaError_t launch_backproject_naive(const DevJob *d_jobs, int job, int nu, int nv, cudaStream_t st);

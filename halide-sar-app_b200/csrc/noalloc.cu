@@ -127,10 +127,8 @@ __global__ void init_items_kernel(WorkItem *items, int ntiles, int nitems, RowIt
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < nitems) items[t] = WorkItem{0, t % ntiles, t / ntiles};
     if (t < npulses) rows[t] = RowItem{0, t};
-    if (t == 0) {
-        *counter = 0;
-        *split_list = 0;
-    }
+    if (t < kBpCounterBytes / (int)sizeof(int)) counter[t] = 0;
+    if (t == 0) *split_list = 0;
 }
 
 __global__ void status_kernel(const JobScalars *sc, int *status) { *status = sc->status; }
@@ -190,7 +188,7 @@ extern "C" int sarbp_backprojection_noalloc(const sarbp_job *job, void *cuda_str
     const size_t o_items = o; o = align_up(o + nitems * sizeof(WorkItem), 256);
     const size_t o_split = o; o = align_up(o + sizeof(int), 256);
     const size_t o_rows = o;  o = align_up(o + P * sizeof(RowItem), 256);
-    const size_t o_cnt = o;   o = align_up(o + sizeof(int), 256);
+    const size_t o_cnt = o;   o = align_up(o + kBpCounterBytes, 256);
     const size_t o_qp = o;    o = align_up(o + P * (N + 1) * sizeof(float4), 256);
     const size_t o_filt = o;  o = align_up(o + S * sizeof(float), 256);
     const size_t o_ws = o;    o = align_up(o + S * sizeof(float), 256);
@@ -279,6 +277,7 @@ extern "C" int sarbp_backprojection_noalloc(const sarbp_job *job, void *cuda_str
     const int occ = bp_max_active_blocks(L);
     if (occ < 1) return fail(SARBP_ERR_CUDA, "no-alloc: backprojection kernel does not fit on an SM");
     L.grid = (int)std::min<long long>((long long)occ * num_sms, (long long)nitems);
+    L.deal.how = kDealItems;  // one job: its parts differ by a pulse at most
     e = launch_backproject(L, d_job, d_items, (int)nitems, d_cnt, st);
     if (e == cudaSuccess && nsplit > 1) e = launch_combine_parts(d_job, d_split, 1, (long long)j.nu * j.nv, num_sms, st);
     if (e == cudaSuccess && j.out_u8) e = launch_batch_u8(d_job, 1, (long long)j.nu * j.nv, st);

@@ -267,6 +267,7 @@ BpLaunch default_launch(const sarbp_opts *opts, int num_sms) {
     L.stage_cap = 2048;
     L.cmax = 64;
     L.persistent = 1;
+    L.deal = BpDeal{kDealNone, 0, 0};
     L.parts = 0;
     if (opts) {
         if (opts->tile_x > 0 && opts->tile_y > 0) {
@@ -486,7 +487,7 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
     const size_t o_tiles = align_up(o_items + items.size() * sizeof(WorkItem), 256);
     const size_t o_split = align_up(o_tiles + tiles.size() * sizeof(WorkItem), 256);
     const size_t o_cnt = align_up(o_split + split.size() * sizeof(int), 256);
-    const size_t meta_bytes = o_cnt + 256 * (size_t)(slabs ? slabs->nslabs : 1);
+    const size_t meta_bytes = o_cnt + (slabs ? kBpCounterBytes * (size_t)slabs->nslabs : (size_t)kBpDealBytes);
     if (for_graph && (host_meta_.cap < meta_bytes || meta_.cap < meta_bytes))
         return fail(SARBP_ERR_STATE, "graph capture needs a prior run of the same jobs");
     // the previous batch's descriptor copy must have left host_meta_
@@ -646,7 +647,7 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
                 BpLaunch Lg = L;
                 Lg.persistent = 0;
                 Lg.grid = n;
-                if (e == cudaSuccess) e = launch_backproject(Lg, d_jobs, d_items + first, n, d_cnt + 64 * g, sg);
+                if (e == cudaSuccess) e = launch_backproject(Lg, d_jobs, d_items + first, n, d_cnt + kBpCounterBytes / 4 * g, sg);
                 if (e != cudaSuccess) return cuda_fail(e, "slab launch");
                 dev_->launches += 2;
             }
@@ -669,6 +670,22 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
             const int occ = bp_max_active_blocks(L);
             if (occ < 1) return fail(SARBP_ERR_CUDA, "backprojection kernel does not fit on an SM");
             L.grid = std::min<long long>((long long)occ * dev_->num_sms, (long long)items.size());
+            // sorted longest first: equal when the ends differ by a pulse at
+            // most (parts of one job).  Uneven lists: even shares of pulses
+            // over the last three rounds of the longest item
+            const int longest = item_pulses(items.front()), shortest = item_pulses(items.back());
+            if (longest - shortest <= 1) {
+                L.deal.how = kDealItems;
+            } else {
+                const long long zone_work = 3ll * longest * dev_->num_sms;
+                long long total = 0, zone = (long long)items.size();
+                for (size_t i = items.size(); i-- > 0;) {
+                    total += item_pulses(items[i]);
+                    if (total <= zone_work) zone = (long long)i;
+                }
+                // an SM's pulses are counted in one word
+                if (total < (1ll << 31)) L.deal = BpDeal{kDealPulses, (int)zone, total};
+            }
         }
         e = launch_backproject(L, d_jobs, d_items, (int)items.size(), d_cnt, st);
         if (e != cudaSuccess) return cuda_fail(e, "backprojection launch");

@@ -1,0 +1,75 @@
+"""The backprojection's work list: persistent CTAs that claim further items
+(with even shares of the end of the list) form the same image, bit for bit,
+as one CTA per tile; GPU tests."""
+import numpy as np
+import pytest
+
+import sarbp_b200 as sb
+from sarbp_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch():
+    return pytest.importorskip("torch")
+
+
+def _cfg(P, seed, **kw):
+    c = dict(P=P, S=96, f0=9.6e9, df=1.5e6, R0=4e3, dep=35.0, span=3.0, nscat=5, half=10.0, clutter=0, snr=20.0,
+             n=32, extent=20.0, taylor=20, upsample=2, db=(-40.0, 0.0), seed=seed)
+    c.update(kw)
+    return c
+
+
+class _Job:
+    """A device-resident job of nu x nv pixels at 0.3 m."""
+
+    def __init__(self, torch, nu, nv, P, seed, precise=False):
+        d = synth.make_from(_cfg(P, seed))
+        t = lambda a, k: torch.from_numpy(np.ascontiguousarray(a, k)).cuda()
+        self.a = [t(d["phs"].view(np.float32), np.float32), t(d["k_r"], np.float32), t(d["pos"], np.float32),
+                  t((np.arange(nu) - nu // 2) * 0.3, np.float64), t((np.arange(nv) - nv // 2) * 0.3, np.float64),
+                  t(d["k_r"], np.float64), t(d["pos"], np.float64)]
+        self.out = torch.full((nv, nu, 2), -7.0, dtype=torch.float64, device="cuda")
+        self.u8 = torch.zeros((nv, nu), dtype=torch.uint8, device="cuda")
+        p = [x.data_ptr() for x in self.a]
+        self.job = sb.make_job(d["S"], P, d["N_fft"], 20, nu, nv, d["delta_r"], p[0], p[1], p[2],
+                               self.out.data_ptr(), u=p[3], v=p[4], u_hat=d["u_hat"], v_hat=d["v_hat"], k_r64=p[5],
+                               pos64=p[6], out_u8=self.u8.data_ptr(), dB_min=-40.0, dB_max=0.0,
+                               precision=sb.PREC_PRECISE if precise else sb.PREC_COMPAT)
+
+    def run(self, ctx, jobs=None, **tune):
+        ctx.run_jobs(jobs or [self.job], **tune)
+        ctx.synchronize()
+        return self.out.cpu().numpy().copy(), self.u8.cpu().numpy().copy()
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    with sb.Context(0) as c:
+        yield c
+
+
+# tiles: one; all resident (3 x 148) less and more one; between one and two
+# rounds; above two rounds; pulses: fewer and more than a chunk, odd
+@pytest.mark.parametrize("tx,ty,P", [(1, 1, 3), (443, 1, 65), (37, 12, 40), (89, 5, 129), (23, 32, 70), (33, 31, 11)])
+def test_claimed_items_equal_one_cta_per_tile(ctx, torch, tx, ty, P):
+    j = _Job(torch, 32 * tx - 5, 32 * ty - 3, P, seed=tx)
+    want = j.run(ctx, persistent=2, pulse_parts=1)
+    assert np.isfinite(want[0]).all() and np.abs(want[0]).max() > 0
+    got = j.run(ctx, pulse_parts=1)
+    assert np.array_equal(want[0], got[0]) and np.array_equal(want[1], got[1])
+
+
+@pytest.mark.parametrize("precise", [False, True])
+def test_uneven_list_equals_each_job_alone(ctx, torch, precise):
+    sizes = [(700, 500, 211), (96, 96, 17), (513, 130, 90), (64, 1000, 64), (40, 30, 1), (300, 300, 150)]
+    jobs = [_Job(torch, nu, nv, P, seed=i, precise=precise) for i, (nu, nv, P) in enumerate(sizes)]
+    alone = [j.run(ctx) for j in jobs]
+    for j in jobs:
+        j.out.fill_(-7.0)
+        j.u8.fill_(0)
+    jobs[0].run(ctx, jobs=[j.job for j in jobs])
+    for j, (img, u8) in zip(jobs, alone):
+        assert np.array_equal(img, j.out.cpu().numpy()) and np.array_equal(u8, j.u8.cpu().numpy())
