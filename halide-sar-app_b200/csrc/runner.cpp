@@ -30,14 +30,14 @@ struct JobLayout {
 // tile kernel the tile table, per-(tile, pulse) records and final phases,
 // and for a job formed in nsplit > 1 pulse parts one partial image per part.
 JobLayout layout_of(const sarbp_job &j, size_t base, int tile_x, int tile_y, bool rc_only, bool naive,
-                    bool resident = false, int nsplit = 1) {
+                    bool resident = false, int nsplit = 1, bool q_direct = false) {
     JobLayout L;
     const size_t P = (size_t)j.npulses, N = (size_t)j.n_fft, S = (size_t)j.nsamples;
     const bool tiles = !rc_only && !naive;
     const size_t ntiles =
         tiles ? (size_t)((j.nu + tile_x - 1) / tile_x) * (size_t)((j.nv + tile_y - 1) / tile_y) : 0;
     size_t o = base;
-    L.Q = o;      o = align_up(o + (rc_only ? P * N * sizeof(float2) : 0), 256);
+    L.Q = o;      o = align_up(o + (rc_only && !q_direct ? P * N * sizeof(float2) : 0), 256);
     L.Qp = o;     o = align_up(o + (rc_only || resident ? 0 : P * (N + 1) * sizeof(float4)), 256);
     L.filt = o;   o = align_up(o + S * sizeof(float), 256);
     L.wS = o;     o = align_up(o + S * sizeof(float), 256);
@@ -49,6 +49,20 @@ JobLayout layout_of(const sarbp_job &j, size_t base, int tile_x, int tile_y, boo
     L.parts = o;  o = align_up(o + (tiles && nsplit > 1 ? (size_t)nsplit * j.nu * j.nv * sizeof(float2) : 0), 256);
     L.end = o;
     return L;
+}
+
+// Whether the range-compression kernels may store a job's profiles at q.
+bool writable_profiles(const void *q, const sarbp_job &j, int device) {
+    if (reinterpret_cast<uintptr_t>(q) % sizeof(float2)) return false;
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (a.type != cudaMemoryTypeDevice || a.device != device) return false;
+    const char *q0 = static_cast<const char *>(q), *x0 = reinterpret_cast<const char *>(j.phs);
+    const size_t nq = (size_t)j.npulses * j.n_fft * sizeof(float2), nx = (size_t)j.npulses * j.nsamples * sizeof(float2);
+    return q0 + nq <= x0 || x0 + nx <= q0;
 }
 
 int precision_of(const sarbp_job &j, const sarbp_opts *o) {
@@ -384,6 +398,10 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         cudaError_t e = cudaEventCreateWithFlags(&meta_done_, cudaEventDisableTiming);
         if (e != cudaSuccess) return cuda_fail(e, "cudaEventCreate");
     }
+    // Range profiles go straight to a q_out that the kernels can write (device
+    // memory of this device, aligned for complex stores, apart from the phase
+    // history they are formed from); else through scratch and a copy.
+    const bool q_direct = rc_only && writable_profiles(q_out, jobs[0], dev_->device);
     // ---- pulse parts (row slabs come only for images of 2^18 pixels and
     // more without a requested part count, which pulse_parts never splits) ----
     std::vector<int> nsplit(njobs, 1);
@@ -395,7 +413,7 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
     std::vector<JobLayout> lay(njobs);
     for (int i = 0; i < njobs; ++i) {
         lay[i] = layout_of(jobs[i], off, L.tile_x, L.tile_y, rc_only, prec[i] == SARBP_PREC_NAIVE, resident(i),
-                           nsplit[i]);
+                           nsplit[i], q_direct);
         off = lay[i].end;
     }
     // work buffer of the four-step range compression (N_fft above
@@ -506,7 +524,7 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         const sarbp_job &j = jobs[i];
         DevJob &dj = hj[i];
         describe_job(j, prec[i], L.tile_x, L.tile_y, dj);
-        dj.Q = reinterpret_cast<float2 *>(sbase + lay[i].Q);
+        dj.Q = q_direct ? static_cast<float2 *>(q_out) : reinterpret_cast<float2 *>(sbase + lay[i].Q);
         dj.Qp = rc_only ? nullptr
                 : resident(i) ? const_cast<float4 *>(resident_qp[i])
                               : reinterpret_cast<float4 *>(sbase + lay[i].Qp);
@@ -613,9 +631,11 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
     }
     if ((e = rec(2)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
     if (rc_only) {
-        e = cudaMemcpyAsync(q_out, hj[0].Q, (size_t)jobs[0].npulses * jobs[0].n_fft * sizeof(float2),
-                            cudaMemcpyDeviceToDevice, st);
-        if (e != cudaSuccess) return cuda_fail(e, "copying range profiles");
+        if (!q_direct) {
+            e = cudaMemcpyAsync(q_out, hj[0].Q, (size_t)jobs[0].npulses * jobs[0].n_fft * sizeof(float2),
+                                cudaMemcpyDeviceToDevice, st);
+            if (e != cudaSuccess) return cuda_fail(e, "copying range profiles");
+        }
         if ((e = copy_status()) != cudaSuccess) return cuda_fail(e, "copying job status");
         return SARBP_OK;
     }
