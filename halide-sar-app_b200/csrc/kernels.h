@@ -25,7 +25,7 @@ cudaError_t init_range_compress_attributes();
 // work_rows rows of N_fft complex values (rows go through it work_rows at a
 // time; rc_work_rows(logN) rows, rc_work_bytes(logN) bytes, is about
 // 256 MB); tw1 and tw2 are the tables of logN / 2 and logN - logN / 2, twN
-// the W_N table.
+// the W_N^(n2 k1) table (logN 15..17).
 int rc_work_rows(int logN);
 size_t rc_work_bytes(int logN);
 cudaError_t launch_range_compress_large(int logN, const DevJob *d_jobs, const RowItem *d_rows, int nrows,
