@@ -173,20 +173,16 @@ int sarbp_accum::start() {
     b.recs = reinterpret_cast<PulseRec *>(dptr(lay.recs));
     b.acc = nullptr;
     b.chunked = 0;
-    cudaError_t e = launch_store_job(b, d_job(), s);
-    // windows, filter, pulse table, k_c (clears max|z| and status)
-    if (e == cudaSuccess) {
-        launch_prep(d_job(), 1, s);
-        e = cudaGetLastError();
-    }
+    b.host_status = nullptr;
+    // windows, filter, pulse table, k_c (clears max|z| and status), lists
     auto *items = reinterpret_cast<WorkItem *>(dptr(lay.items));
     auto *rows = reinterpret_cast<RowItem *>(dptr(lay.rows));
-    if (e == cudaSuccess) e = launch_fill_items(items, ntiles, rows, C, s);
+    cudaError_t e = launch_prep_single(b, SingleLists{d_job(), items, ntiles, ntiles, rows, C, nullptr, 0}, s);
     // tile table and final phase per pixel (no records: those come per chunk)
     if (e == cudaSuccess) e = launch_tile_setup(d_job(), items, ntiles, L.tile_x * L.tile_y, s, 0);
     if (e == cudaSuccess) e = cudaMemsetAsync(dptr(lay.acc), 0, (size_t)npix * sizeof(float2), s);
     if (e != cudaSuccess) return cuda_fail(e, "pulse-chunked job: set-up launches");
-    ctx->dev.launches += 4;
+    ctx->dev.launches += 2;
     return SARBP_OK;
 }
 
@@ -205,14 +201,12 @@ int sarbp_accum::add(int q0, int n, const float *phs_rows, cudaEvent_t rc_done) 
     auto *items = reinterpret_cast<const WorkItem *>(dptr(lay.items));
     auto *rows = reinterpret_cast<const RowItem *>(dptr(lay.rows));
     int *cnt = reinterpret_cast<int *>(dptr(lay.cnt));
-    cudaError_t e = launch_chunk_tables(base.pulse, base.wP, P, q0, n, c.pulse, c.wP, s);
-    if (e == cudaSuccess) e = launch_store_job(c, d_job(), s);
+    cudaError_t e = launch_chunk_setup(c, d_job(), base.pulse, base.wP, P, q0, cnt, s);
     if (e == cudaSuccess)
         e = range_compress_rows(&ctx->dev, logN, d_job(), rows, n, 1, reinterpret_cast<float2 *>(dptr(lay.work)),
                                 lay.work_rows, s);
     if (e == cudaSuccess && rc_done) e = cudaEventRecord(rc_done, s);
     if (e == cudaSuccess) e = launch_tile_records(d_job(), items, ntiles, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, kBpCounterBytes, s);
     if (e != cudaSuccess) return cuda_fail(e, "pulse-chunked job: chunk launches");
     BpLaunch Lc = L;
     const int occ = bp_max_active_blocks(Lc);
@@ -221,7 +215,7 @@ int sarbp_accum::add(int q0, int n, const float *phs_rows, cudaEvent_t rc_done) 
     Lc.deal.how = kDealItems;  // one chunk's pulses in every tile
     e = launch_backproject(Lc, d_job(), items, ntiles, cnt, s);
     if (e != cudaSuccess) return cuda_fail(e, "pulse-chunked job: backprojection launch");
-    ctx->dev.launches += 5;
+    ctx->dev.launches += 4;
     for (int q = q0; q < q0 + n; ++q) added[q] = 1;
     nadded += n;
     return SARBP_OK;
@@ -342,10 +336,10 @@ int sarbp_accum_finalize(sarbp_accum *acc) {
     DevJob f = acc->base;
     f.acc = reinterpret_cast<float2 *>(acc->dptr(acc->lay.acc));
     JobScalars *sc = reinterpret_cast<JobScalars *>(acc->dptr(acc->lay.sc));
-    cudaError_t e = launch_store_job(f, acc->d_job(), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(&sc->maxabs, 0, sizeof(sc->maxabs), s);
-    if (e == cudaSuccess) e = launch_finalize(acc->d_job(), acc->npix, acc->ctx->dev.num_sms, s);
-    int nl = 2;
+    // max|z| is clear since the set-up or the reset; the u8 kernel reads the
+    // last chunk's descriptor, which names the same image
+    cudaError_t e = launch_finalize(f, acc->npix, acc->ctx->dev.num_sms, s);
+    int nl = 1;
     if (e == cudaSuccess && acc->job.out_u8) {
         e = launch_batch_u8(acc->d_job(), 1, acc->npix, s);
         ++nl;

@@ -44,8 +44,9 @@
 // Claims::next).
 // A job with too few tiles to fill the resident CTAs has each
 // tile split into nsplit items over consecutive pulse ranges; each stores
-// its sums into its own slice of the job's parts buffer (plain stores, no
-// atomics), and the combine kernel adds the slices in a fixed order.
+// its sums into its own slice of the job's parts buffer, and the CTA that
+// completes a tile's last part (a counter per tile) adds the slices in part
+// order, so that the image does not depend on which CTA that is.
 //
 // Naive kernel: the same quantity with plain FP32 range |pos| - |r - pos|
 // and phase k_c * dr per pixel*pulse; kept as the precision-study baseline.
@@ -66,6 +67,7 @@ constexpr int kConsumers = 256;                   // consumer threads (8 warps)
 constexpr int kThreads = kConsumers + 32;         // plus one producer warp
 constexpr int kBarFull0 = 1;                      // named barriers 1, 2: chunk staged
 constexpr int kBarEmpty0 = 3;                     // named barriers 3, 4: chunk consumed
+constexpr int kBarConsumers = 5;                  // consumers among themselves
 
 __device__ __forceinline__ void bar_sync(int id) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(kThreads) : "memory");
@@ -299,13 +301,15 @@ struct __align__(16) ItemCtx {
     const double *r, *u, *v;
     const float2 *fin;  // [nv][nu] final phases
     float2 *sums;       // kItemAcc: partial image; kItemPart: the part's slice
+    const float2 *parts;  // kItemPart: all slices, and the tile's count of parts done
+    int *done;
     double2 *out;
     JobScalars *sc;
     float w0[3], kcf;
     float ilk;  // range bins per radian of Delta
-    int nu, nv, tx0, ty0, flags;
+    int nu, nv, tx0, ty0, flags, nsplit;
 };
-constexpr int kItemTransposed = 1, kItemAcc = 2, kItemPart = 4, kItemMax = 8, kItemTooWide = 16;
+constexpr int kItemTransposed = 1, kItemAcc = 2, kItemPart = 4, kItemMax = 8;
 // An item's slot is rewritten four items later, when the consumers have long
 // passed its epilogue (the producer is at most two chunks ahead).
 constexpr int kCtxSlots = 4;
@@ -319,6 +323,7 @@ struct TileSmem {
     uint64_t *mbar_win;  // [2]
     int4 *s_chunk;       // [2] what each half holds (see below)
     ItemCtx *ctx;        // [kCtxSlots] constants of the items in flight
+    int *s_last;         // whether this CTA completed its tile's parts
 };
 
 struct TileShape {
@@ -476,8 +481,8 @@ struct Claims {
 };
 
 // An item's constants for the consumers.
-__device__ __forceinline__ void fill_ctx(ItemCtx &c, const DevJob &jb, const WorkItem &wi, int flags) {
-    const TileInfo &t = jb.tiles[wi.tile];
+__device__ __forceinline__ void fill_ctx(ItemCtx &c, const DevJob &jb, const WorkItem &wi) {
+    TileInfo &t = jb.tiles[wi.tile];
     const double k_c = jb.sc->k_c;
     for (int d = 0; d < 3; ++d) {
         c.rc[d] = t.rc[d];
@@ -492,6 +497,9 @@ __device__ __forceinline__ void fill_ctx(ItemCtx &c, const DevJob &jb, const Wor
     c.out = jb.out;
     c.sc = jb.sc;
     c.sums = jb.nsplit > 1 ? jb.parts + (long long)wi.part * ((long long)jb.nu * jb.nv) : jb.acc;
+    c.parts = jb.parts;
+    c.done = &t.parts_done;
+    c.nsplit = jb.nsplit;
     c.kcf = (float)k_c;
     c.ilk = (float)(jb.inv_lsr / k_c);
     c.nu = jb.nu;
@@ -499,8 +507,8 @@ __device__ __forceinline__ void fill_ctx(ItemCtx &c, const DevJob &jb, const Wor
     c.tx0 = (wi.tile % jb.tiles_x) * jb.tile_x;
     c.ty0 = (wi.tile / jb.tiles_x) * jb.tile_y;
     // only the u8 image uses max|z|
-    c.flags = flags | (t.transposed ? kItemTransposed : 0) |
-              (jb.nsplit > 1 ? kItemPart : jb.acc ? kItemAcc : jb.out_u8 ? kItemMax : 0);
+    c.flags = (t.transposed ? kItemTransposed : 0) |
+              (jb.nsplit > 1 ? kItemPart : jb.acc ? kItemAcc : 0) | (jb.out_u8 && !jb.acc ? kItemMax : 0);
 }
 
 // Producer warp: the same barrier sequence as the consumers.
@@ -552,7 +560,7 @@ __device__ __forceinline__ void producer_loop(const DevJob *__restrict__ jobs,
                 stage_records(jb, wi.tile, lane, p0, nc, b, sm);
             }
             if (c == 0 && more && lane == 0)
-                fill_ctx(sm.ctx[n & (kCtxSlots - 1)], jb, wi, sh.C < 1 ? kItemTooWide : 0);
+                fill_ctx(sm.ctx[n & (kCtxSlots - 1)], jb, wi);
             if (c < sh.nchunks)
                 ok = stage_windows(jb, lane, pb + c * sh.C, nc, b, sh, stage_cap, cmax, sm, uses, mode) && ok;
             if (lane == 0)
@@ -563,7 +571,8 @@ __device__ __forceinline__ void producer_loop(const DevJob *__restrict__ jobs,
             bar_arrive(kBarFull0 + b);
         }
         if (!more) break;
-        if (!ok && lane == 0) atomicOr(&jb.sc->status, kStatusTimeout);
+        if (!ok && lane == 0) report_status(jb, kStatusTimeout);
+        if (sh.C < 1 && lane == 0) report_status(jb, kStatusTileTooWide);
     }
     // the consumers' arrival on the last chunk before the end's empty turn
     if (g >= 2) bar_sync(kBarEmpty0 + (g & 1));
@@ -666,35 +675,57 @@ __device__ __forceinline__ void consumer_loop(int stage_cap, int cmax, const Til
         bar_arrive(kBarEmpty0 + b);
         if (!(done.w & kChunkLast)) continue;
         // ---- final phase, row flip (backprojection.cpp:130-138), max|z|;
-        // a pulse part stores its sums into its slice, a pulse chunk adds
-        // them to the partial image instead; loads before the first store ----
+        // a pulse part stores its sums into its slice and the tile's last part
+        // goes on with the slices' sum, a pulse chunk adds its sums to the
+        // partial image instead; loads before the first store ----
         const ItemCtx &it = sm.ctx[done.x];
-        if ((it.flags & kItemTooWide) && tid == 0) atomicOr(&it.sc->status, kStatusTileTooWide);
-        const bool has_sums = (it.flags & (kItemPart | kItemAcc)) != 0;
-        float2 in[PPT];  // final phases, or the partial image so far
+        float2 sum[PPT], in[PPT];  // the item's sums; final phases, or the partial image so far
+        long long at[PPT];         // pixel, -1 outside the image
 #pragma unroll
         for (int k = 0; k < PPT; ++k) {
             int ix, iy;
             pixel_of(it, k, ix, iy);
-            in[k] = make_float2(0.0f, 0.0f);
-            if (ix < it.nu && iy < it.nv && !(it.flags & kItemPart))
-                in[k] = (has_sums ? it.sums : it.fin)[(long long)iy * it.nu + ix];
+            at[k] = ix < it.nu && iy < it.nv ? (long long)iy * it.nu + ix : -1;
+            sum[k] = make_float2((k & 1) ? arp[k >> 1].y : arp[k >> 1].x, (k & 1) ? aip[k >> 1].y : aip[k >> 1].x);
         }
+        if (it.flags & kItemPart) {
+#pragma unroll
+            for (int k = 0; k < PPT; ++k)
+                if (at[k] >= 0) it.sums[at[k]] = sum[k];
+            __threadfence();  // the slice before the count
+            asm volatile("bar.sync %0, %1;" ::"r"(kBarConsumers), "r"(kConsumers) : "memory");
+            if (tid == 0) *sm.s_last = atomicAdd(it.done, 1) == it.nsplit - 1;
+            asm volatile("bar.sync %0, %1;" ::"r"(kBarConsumers), "r"(kConsumers) : "memory");
+            if (!*sm.s_last) continue;
+            __threadfence();
+            const long long npix = (long long)it.nu * it.nv;
+#pragma unroll
+            for (int k = 0; k < PPT; ++k)
+                if (at[k] >= 0) sum[k] = __ldcg(it.parts + at[k]);
+#pragma unroll 4
+            for (int p = 1; p < it.nsplit; ++p)
+#pragma unroll
+                for (int k = 0; k < PPT; ++k)
+                    if (at[k] >= 0) {
+                        const float2 s = __ldcg(it.parts + p * npix + at[k]);
+                        sum[k].x += s.x;
+                        sum[k].y += s.y;
+                    }
+        }
+        const bool acc = (it.flags & kItemAcc) != 0;
+#pragma unroll
+        for (int k = 0; k < PPT; ++k) in[k] = at[k] >= 0 ? (acc ? it.sums : it.fin)[at[k]] : make_float2(0.0f, 0.0f);
         double zmax = 0.0;
 #pragma unroll
         for (int k = 0; k < PPT; ++k) {
-            int ix, iy;
-            pixel_of(it, k, ix, iy);
-            if (ix >= it.nu || iy >= it.nv) continue;
-            const float ark = (k & 1) ? arp[k >> 1].y : arp[k >> 1].x;
-            const float aik = (k & 1) ? aip[k >> 1].y : aip[k >> 1].x;
-            if (it.flags & kItemPart) {
-                it.sums[(long long)iy * it.nu + ix] = make_float2(ark, aik);
-            } else if (it.flags & kItemAcc) {
-                it.sums[(long long)iy * it.nu + ix] = make_float2(in[k].x + ark, in[k].y + aik);
+            if (at[k] < 0) continue;
+            if (acc) {
+                it.sums[at[k]] = make_float2(in[k].x + sum[k].x, in[k].y + sum[k].y);
             } else {
-                const double zr = (double)fmaf(ark, in[k].x, -aik * in[k].y);
-                const double zi = (double)fmaf(ark, in[k].y, aik * in[k].x);
+                const double zr = (double)fmaf(sum[k].x, in[k].x, -sum[k].y * in[k].y);
+                const double zi = (double)fmaf(sum[k].x, in[k].y, sum[k].y * in[k].x);
+                int ix, iy;
+                pixel_of(it, k, ix, iy);
                 it.out[(long long)(it.nv - 1 - iy) * it.nu + ix] = make_double2(zr, zi);
                 if (it.flags & kItemMax) zmax = fmax(zmax, sqrt(zr * zr + zi * zi));
             }
@@ -719,6 +750,7 @@ __global__ void __launch_bounds__(kThreads, MINB) bp_tile_kernel(const DevJob *_
     extern __shared__ float4 smem[];
     __shared__ int4 s_chunk[2];
     __shared__ ItemCtx s_ctx[kCtxSlots];
+    __shared__ int s_last;
     __shared__ uint64_t mbar[4];
     TileSmem sm;
     sm.stage = smem;
@@ -728,6 +760,7 @@ __global__ void __launch_bounds__(kThreads, MINB) bp_tile_kernel(const DevJob *_
     sm.mbar_win = mbar + 2;
     sm.s_chunk = s_chunk;
     sm.ctx = s_ctx;
+    sm.s_last = &s_last;
     if (threadIdx.x == kConsumers) {
         for (int i = 0; i < 4; ++i)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[i])) : "memory");

@@ -313,6 +313,7 @@ __global__ void __launch_bounds__(kThreadsGeom, GP <= 4 ? 4 : 2)
         // or more, eight lanes span more than the eight 16-byte banks of a
         // shared-memory wavefront and collide.  Run the lanes along the axis
         // with the smaller step (square tiles only).
+        t.parts_done = 0;
         t.transposed = 0;
         if (TX == TY && tx0 + 1 < jb.nu && ty0 + 1 < jb.nv) {
             double x0, y0, z0, x1, y1, z1, x2, y2, z2;
@@ -329,7 +330,7 @@ __global__ void __launch_bounds__(kThreadsGeom, GP <= 4 ? 4 : 2)
         }
         jb.tiles[wi.tile] = t;
         s_tile = t;
-        if (bad) atomicOr(&jb.sc->status, kStatusNonFinite);
+        if (bad) report_status(jb, kStatusNonFinite);
     }
     __syncthreads();
     if (!records) return;  // pulse-chunked jobs form their records per chunk
@@ -346,7 +347,7 @@ __global__ void __launch_bounds__(kThreadsGeom, GP <= 4 ? 4 : 2)
         bad_pulse |= !make_record(jb, t, rk, p, rec);
         recs[p] = rec;
     }
-    if (__any_sync(0xffffffffu, bad_pulse) && lane == 0) atomicOr(&jb.sc->status, kStatusNonFinite);
+    if (__any_sync(0xffffffffu, bad_pulse) && lane == 0) report_status(jb, kStatusNonFinite);
 }
 
 // Records only, for the pulses of one chunk of a pulse-chunked job: the
@@ -368,7 +369,7 @@ __global__ void __launch_bounds__(kThreadsGeom)
         bad_pulse |= !make_record(jb, t, rk, p, rec);
         recs[p] = rec;
     }
-    if (__any_sync(0xffffffffu, bad_pulse) && (threadIdx.x & 31) == 0) atomicOr(&jb.sc->status, kStatusNonFinite);
+    if (__any_sync(0xffffffffu, bad_pulse) && (threadIdx.x & 31) == 0) report_status(jb, kStatusNonFinite);
 }
 
 }  // namespace

@@ -22,8 +22,9 @@ constexpr int kStatusTileTooWide = 1;   // range window of a tile exceeds smem
 constexpr int kStatusNonFinite = 2;     // non-finite pixel or pulse geometry
 constexpr int kStatusNearField = 4;     // pulse closer than the tile radius
 constexpr int kStatusTimeout = 8;       // a bounded wait on an async copy gave up
+constexpr int kStatusWords = 4;         // DevJob::host_status: one word per bit
 
-// per-job words the kernels write; kept contiguous for one status read-back
+// per-job words the kernels write
 struct JobScalars {
     unsigned long long maxabs;  // bits of max |z| (f64, non-negative)
     double k_c;                 // k_r[S/2] by precision mode (prep kernel)
@@ -54,6 +55,7 @@ struct __align__(16) TileInfo {
     int wide;      // 1: records hold w_hat - w0, fin carries exp(-j w0 . d)
     float w0[3];   // unit direction from rc to the mid-aperture antenna (wide tiles)
     int transposed;  // 1: consumer lanes run along y (square tiles; see tile set-up)
+    int parts_done;  // pulse parts of the tile completed (the backprojection counts)
 };
 
 // Per-(tile, pulse) constants (tile geometry kernel -> backprojection):
@@ -94,6 +96,10 @@ struct DevJob {
     PulseRec *recs;       // [tiles][P]
     float2 *fin;          // [nv][nu] exp(+j k_c dr(pixel, P/2)), r-space order
     JobScalars *sc;       // max|z|, k_c, status (written by the kernels)
+    // page-locked host words, one per status bit, or null: the kernels set them
+    // with plain stores beside sc->status (only when something is wrong), so
+    // that no copy has to follow the batch
+    int *host_status;
     // constants
     double delta_r, lsa, lsr, inv_lsr;
     double taylor_F[kMaxTaylorTerms];
@@ -110,8 +116,8 @@ struct DevJob {
     // pulse parts: a job whose tiles leave resident CTAs idle has each tile
     // formed as nsplit items over consecutive pulse ranges (part_range);
     // each item stores its sums into slice `part` of parts ([nsplit][nv][nu],
-    // pixel-row order), and the combine kernel adds the slices in order and
-    // applies the final phase.  nsplit <= 1: one item per tile.
+    // pixel-row order), and the last of a tile's items adds the slices in order
+    // and applies the final phase.  nsplit <= 1: one item per tile.
     int nsplit;
     float2 *parts;
 };
@@ -133,6 +139,14 @@ __host__ __device__ inline void part_range(int P, int nsplit, int part, int &p0,
     p0 = (int)((long long)part * P / nsplit);
     p1 = (int)((long long)(part + 1) * P / nsplit);
 }
+
+#ifdef __CUDACC__
+// Sets status bit `bit` of a job.
+__device__ __forceinline__ void report_status(const DevJob &jb, int bit) {
+    atomicOr(&jb.sc->status, bit);
+    if (jb.host_status) *reinterpret_cast<volatile int *>(jb.host_status + (__ffs(bit) - 1)) = 1;
+}
+#endif
 
 // one row of a batched range-compression launch
 struct RowItem {

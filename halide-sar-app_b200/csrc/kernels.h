@@ -14,6 +14,19 @@ namespace sarbp {
 
 // prep.cu
 void launch_prep(const DevJob *d_jobs, int njobs, cudaStream_t st);
+// One job: its descriptor goes to `job`, its work items (part-major: items
+// [0, ntiles) are part 0 of each tile, the tile list of the geometry kernels)
+// and rows [0, nrows) are listed, and counters[0 .. ncounters) cleared.
+struct SingleLists {
+    DevJob *job;
+    WorkItem *items;
+    int ntiles, nitems;
+    RowItem *rows;
+    int nrows;
+    int *counters;
+    int ncounters;
+};
+cudaError_t launch_prep_single(const DevJob &job, const SingleLists &lists, cudaStream_t st);
 
 // range_compress.cu
 int twiddle_table_size(int logN);
@@ -73,15 +86,11 @@ cudaError_t launch_tile_records(const DevJob *d_jobs, const WorkItem *d_items, i
 
 
 // accum_kernels.cu (pulse-chunked jobs)
-cudaError_t launch_store_job(const DevJob &dj, DevJob *d_dst, cudaStream_t st);
-cudaError_t launch_chunk_tables(const double4 *pulse, const float *wP, int P, int q0, int n, double4 *pulse_c,
-                                float *wP_c, cudaStream_t st);
-cudaError_t launch_finalize(const DevJob *d_job, long long npix, int num_sms, cudaStream_t st);
-cudaError_t launch_fill_items(WorkItem *items, int ntiles, RowItem *rows, int nrows, cudaStream_t st);
-// jobs d_list[0 .. nlist) of d_jobs, formed in pulse parts: sum of the parts
-// times the final phase into out (row flip), max |z|
-cudaError_t launch_combine_parts(const DevJob *d_jobs, const int *d_list, int nlist, long long max_pixels,
-                                 int num_sms, cudaStream_t st);
+// a chunk's descriptor to d_dst, its windows and pulse table gathered into
+// job.wP and job.pulse, the backprojection's counters cleared
+cudaError_t launch_chunk_setup(const DevJob &job, DevJob *d_dst, const double4 *pulse, const float *wP, int P, int q0,
+                               int *counters, cudaStream_t st);
+cudaError_t launch_finalize(const DevJob &job, long long npix, int num_sms, cudaStream_t st);
 
 // resize.cu (the reference's data/resize.py resampling)
 struct ResizePlan {

@@ -116,21 +116,6 @@ int scratch_for_device(int dev, cudaStream_t st, void **addr, int *num_sms) {
     return SARBP_OK;
 }
 
-__global__ void store_job_kernel(DevJob dj, DevJob *dst) { *dst = dj; }
-
-// work items (0, t, s) for the job's tiles and pulse parts (part 0 of every
-// tile first, which the tile-geometry kernel takes as its tile list),
-// range-compression rows (0, p), the persistent launch counter and the
-// combine kernel's job list
-__global__ void init_items_kernel(WorkItem *items, int ntiles, int nitems, RowItem *rows, int npulses,
-                                  int *counter, int *split_list) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < nitems) items[t] = WorkItem{0, t % ntiles, t / ntiles};
-    if (t < npulses) rows[t] = RowItem{0, t};
-    if (t < kBpCounterBytes / (int)sizeof(int)) counter[t] = 0;
-    if (t == 0) *split_list = 0;
-}
-
 __global__ void status_kernel(const JobScalars *sc, int *status) { *status = sc->status; }
 
 }  // namespace
@@ -186,7 +171,6 @@ extern "C" int sarbp_backprojection_noalloc(const sarbp_job *job, void *cuda_str
     const size_t o_sc = o;    o = align_up(o + sizeof(JobScalars), 256);
     const size_t o_job = o;   o = align_up(o + sizeof(DevJob), 256);
     const size_t o_items = o; o = align_up(o + nitems * sizeof(WorkItem), 256);
-    const size_t o_split = o; o = align_up(o + sizeof(int), 256);
     const size_t o_rows = o;  o = align_up(o + P * sizeof(RowItem), 256);
     const size_t o_cnt = o;   o = align_up(o + kBpCounterBytes, 256);
     const size_t o_qp = o;    o = align_up(o + P * (N + 1) * sizeof(float4), 256);
@@ -260,16 +244,11 @@ extern "C" int sarbp_backprojection_noalloc(const sarbp_job *job, void *cuda_str
     int *d_cnt = reinterpret_cast<int *>(sb + o_cnt);
     const float2 *d_tw = reinterpret_cast<const float2 *>(sb + twiddle_offset(logN));
     RowItem *d_rows = reinterpret_cast<RowItem *>(sb + o_rows);
-    int *d_split = reinterpret_cast<int *>(sb + o_split);
 
     // ---- launches (the prep kernel clears the job's scalars) ----
-    store_job_kernel<<<1, 1, 0, st>>>(dj, d_job);
-    const size_t nfill = nitems > P ? nitems : P;
-    init_items_kernel<<<(int)((nfill + 255) / 256), 256, 0, st>>>(d_items, (int)ntiles, (int)nitems, d_rows,
-                                                                  j.npulses, d_cnt, d_split);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_fail(e, "no-alloc set-up launches");
-    launch_prep(d_job, 1, st);
+    e = launch_prep_single(dj, SingleLists{d_job, d_items, (int)ntiles, (int)nitems, d_rows, j.npulses, d_cnt,
+                                           kBpCounterBytes / (int)sizeof(int)}, st);
+    if (e != cudaSuccess) return cuda_fail(e, "no-alloc set-up launch");
     e = launch_range_compress(logN, d_job, d_rows, j.npulses, 1, d_tw, st);
     if (e == cudaSuccess) e = launch_tile_setup(d_job, d_items, (int)ntiles, L0.tile_x * L0.tile_y, st);
     if (e != cudaSuccess) return cuda_fail(e, "no-alloc range compression / geometry launch");
@@ -279,7 +258,6 @@ extern "C" int sarbp_backprojection_noalloc(const sarbp_job *job, void *cuda_str
     L.grid = (int)std::min<long long>((long long)occ * num_sms, (long long)nitems);
     L.deal.how = kDealItems;  // one job: its parts differ by a pulse at most
     e = launch_backproject(L, d_job, d_items, (int)nitems, d_cnt, st);
-    if (e == cudaSuccess && nsplit > 1) e = launch_combine_parts(d_job, d_split, 1, (long long)j.nu * j.nv, num_sms, st);
     if (e == cudaSuccess && j.out_u8) e = launch_batch_u8(d_job, 1, (long long)j.nu * j.nv, st);
     if (e == cudaSuccess && status) {
         status_kernel<<<1, 1, 0, st>>>(dj.sc, status);

@@ -88,11 +88,8 @@ __device__ void image_frame(const DevJob &jb, double (&E)[3][3]) {
     E[1][2] = 0.0;
 }
 
-__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
-    prep_kernel(const DevJob *__restrict__ jobs) {
-    const DevJob &jb = jobs[blockIdx.x / kCluster];
-    const int what = blockIdx.y;
-    const int first = (blockIdx.x % kCluster) * kPrepThreads + threadIdx.x;  // this thread's first element
+__device__ __forceinline__ void prep_part(const DevJob &jb, int what, int rank) {
+    const int first = rank * kPrepThreads + threadIdx.x;  // this thread's first element
     constexpr int kStride = kCluster * kPrepThreads;
     if (what == 0 || what == 1) {
         const int num = what == 0 ? jb.S : jb.P;
@@ -124,6 +121,8 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
             if (first == 0) {
                 jb.sc->maxabs = 0ull;
                 jb.sc->status = 0;
+                if (jb.host_status)
+                    for (int k = 0; k < kStatusWords; ++k) *reinterpret_cast<volatile int *>(jb.host_status + k) = 0;
                 const int h = jb.S / 2;  // k_c = k_r[S/2] (backprojection.cpp:123)
                 jb.sc->k_c = (jb.precision == SARBP_PREC_PRECISE_ && jb.k_r64) ? jb.k_r64[h]
                                                                                : (double)jb.k_r32[h];
@@ -178,10 +177,36 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
     }
 }
 
+__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
+    prep_kernel(const DevJob *__restrict__ jobs) {
+    prep_part(jobs[blockIdx.x / kCluster], blockIdx.y, blockIdx.x % kCluster);
+}
+
+// The same for one job whose descriptor comes as a kernel parameter, which
+// also stores it and makes the job's lists: no upload has to come first (the
+// copy and the gaps around it were 15 us of a 256^2 image's 72).
+__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
+    prep_single_kernel(const __grid_constant__ DevJob job, const SingleLists l) {
+    const int i0 = (blockIdx.y * kCluster + blockIdx.x) * kPrepThreads + threadIdx.x;
+    constexpr int kAll = 3 * kCluster * kPrepThreads;
+    constexpr int kWords = sizeof(DevJob) / sizeof(uint32_t);
+    static_assert(sizeof(DevJob) % sizeof(uint32_t) == 0 && kWords <= kAll, "one word a thread");
+    if (i0 < kWords) reinterpret_cast<uint32_t *>(l.job)[i0] = reinterpret_cast<const uint32_t *>(&job)[i0];
+    for (int i = i0; i < l.nitems; i += kAll) l.items[i] = WorkItem{0, i % l.ntiles, i / l.ntiles};
+    for (int i = i0; i < l.nrows; i += kAll) l.rows[i] = RowItem{0, i};
+    for (int i = i0; i < l.ncounters; i += kAll) l.counters[i] = 0;
+    prep_part(job, blockIdx.y, blockIdx.x);
+}
+
 }  // namespace
 
 void launch_prep(const DevJob *d_jobs, int njobs, cudaStream_t st) {
     prep_kernel<<<dim3(njobs * kCluster, 3), kPrepThreads, 0, st>>>(d_jobs);
+}
+
+cudaError_t launch_prep_single(const DevJob &job, const SingleLists &lists, cudaStream_t st) {
+    prep_single_kernel<<<dim3(kCluster, 3), kPrepThreads, 0, st>>>(job, lists);
+    return cudaGetLastError();
 }
 
 }  // namespace sarbp

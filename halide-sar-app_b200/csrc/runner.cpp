@@ -145,6 +145,7 @@ void describe_job(const sarbp_job &j, int prec, int tile_x, int tile_y, DevJob &
     dj.out_u8 = j.out_u8;
     dj.dB_min = j.dB_min;
     dj.dB_max = j.dB_max;
+    dj.host_status = nullptr;
     dj.chunked = 0;
     dj.acc = nullptr;
     dj.nsplit = 1;
@@ -425,7 +426,7 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         work_off = off;
         off = align_up(off + work_bytes, 256);
     }
-    if (for_graph && (scratch_.cap < off || pool_ || status_pin_.cap < njobs * sizeof(JobScalars)))
+    if (for_graph && (scratch_.cap < off || pool_ || status_pin_.cap < njobs * kStatusWords * sizeof(int)))
         return fail(SARBP_ERR_STATE, "graph capture needs a prior run of the same jobs");
     cudaError_t e;
     char *sbase = nullptr;
@@ -451,26 +452,38 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         if (e != cudaSuccess) return cuda_fail(e, "allocating scratch");
         sbase = static_cast<char *>(scratch_.ptr);
     }
-    // status words come back through a pinned copy enqueued behind the batch
-    if (status_pin_.cap < njobs * sizeof(JobScalars)) {
+    // status words, set by the kernels when something is wrong
+    const size_t status_bytes = (size_t)njobs * kStatusWords * sizeof(int);
+    if (status_pin_.cap < status_bytes) {
         if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(e, "synchronising the stream");
-        if ((e = status_pin_.ensure(njobs * sizeof(JobScalars))) != cudaSuccess)
-            return cuda_fail(e, "allocating pinned status words");
+        if ((e = status_pin_.ensure(status_bytes)) != cudaSuccess) return cuda_fail(e, "allocating pinned status words");
+        std::memset(status_pin_.ptr, 0, status_bytes);
     }
-    auto copy_status = [&]() -> cudaError_t {
-        last_njobs_ = njobs;
-        return cudaMemcpyAsync(status_pin_.ptr, sbase, njobs * sizeof(JobScalars), cudaMemcpyDeviceToHost, st);
-    };
-
     // ---- rows grouped by N_fft, work items longest first, one tile-geometry
-    // item per tile, the jobs formed in pulse parts ----
+    // item per tile.  One job alone needs no lists from the host: the set-up
+    // kernel takes its descriptor as a parameter and makes them (rows and
+    // tiles in order, parts one after another) ----
+    const bool single = njobs == 1;
+    struct RowGroup {
+        int logN;
+        size_t first, count;
+    };
+    std::vector<RowGroup> row_groups;
     std::map<int, std::vector<RowItem>> rows;
     std::vector<WorkItem> items, tiles;
-    std::vector<int> naive, split;
+    std::vector<int> naive;
+    size_t nrows_total = 0, nitems = 0, ntile_items = 0;
+    bool any_split = false;
     for (int i = 0; i < njobs; ++i) {
+        const size_t P = (size_t)jobs[i].npulses;
         if (!resident(i)) {  // resident profiles were range-compressed before
-            auto &v = rows[ilog2i(jobs[i].n_fft)];
-            for (int p = 0; p < jobs[i].npulses; ++p) v.push_back(RowItem{i, p});
+            if (single) {
+                row_groups.push_back({ilog2i(jobs[i].n_fft), 0, P});
+                nrows_total = P;
+            } else {
+                auto &v = rows[ilog2i(jobs[i].n_fft)];
+                for (int p = 0; p < jobs[i].npulses; ++p) v.push_back(RowItem{i, p});
+            }
         }
         if (rc_only) continue;
         if (prec[i] == SARBP_PREC_NAIVE) {
@@ -479,9 +492,12 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         }
         const int tx = (jobs[i].nu + L.tile_x - 1) / L.tile_x;
         const int ty = (jobs[i].nv + L.tile_y - 1) / L.tile_y;
+        ntile_items += (size_t)tx * ty;
+        nitems += (size_t)tx * ty * nsplit[i];
+        any_split = any_split || nsplit[i] > 1;
+        if (single) continue;
         for (int s = 0; s < nsplit[i]; ++s)
             for (int t = 0; t < tx * ty; ++t) items.push_back(WorkItem{i, t, s});
-        if (nsplit[i] > 1) split.push_back(i);
     }
     auto item_pulses = [&](const WorkItem &w) {
         int p0, p1;
@@ -490,36 +506,41 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
     };
     std::stable_sort(items.begin(), items.end(),
                      [&](const WorkItem &a, const WorkItem &b) { return item_pulses(a) > item_pulses(b); });
-    if (!split.empty())
+    if (any_split)
         for (const WorkItem &w : items)
             if (w.part == 0) tiles.push_back(w);
-    size_t nrows_total = 0;
-    for (auto &kv : rows) nrows_total += kv.second.size();
+    for (auto &kv : rows) {
+        row_groups.push_back({kv.first, nrows_total, kv.second.size()});
+        nrows_total += kv.second.size();
+    }
 
     // ---- meta block: [DevJob][RowItem...][WorkItem...][tile WorkItem...]
-    // [split job...][counter] (the tile list only when a job is split: the
-    // work items are then not one per tile) ----
+    // [counters] (the tile list only when a job of several is split: the work
+    // items are then not one per tile) ----
     const size_t o_jobs = 0;
     const size_t o_rows = align_up(o_jobs + (size_t)njobs * sizeof(DevJob), 256);
     const size_t o_items = align_up(o_rows + nrows_total * sizeof(RowItem), 256);
-    const size_t o_tiles = align_up(o_items + items.size() * sizeof(WorkItem), 256);
-    const size_t o_split = align_up(o_tiles + tiles.size() * sizeof(WorkItem), 256);
-    const size_t o_cnt = align_up(o_split + split.size() * sizeof(int), 256);
-    const size_t meta_bytes = o_cnt + (slabs ? kBpCounterBytes * (size_t)slabs->nslabs : (size_t)kBpDealBytes);
-    if (for_graph && (host_meta_.cap < meta_bytes || meta_.cap < meta_bytes))
+    const size_t o_tiles = align_up(o_items + nitems * sizeof(WorkItem), 256);
+    const size_t o_cnt = align_up(o_tiles + tiles.size() * sizeof(WorkItem), 256);
+    const size_t cnt_bytes = slabs ? kBpCounterBytes * (size_t)slabs->nslabs : (size_t)kBpDealBytes;
+    const size_t meta_bytes = o_cnt + cnt_bytes;
+    if (for_graph && ((!single && host_meta_.cap < meta_bytes) || meta_.cap < meta_bytes))
         return fail(SARBP_ERR_STATE, "graph capture needs a prior run of the same jobs");
-    // the previous batch's descriptor copy must have left host_meta_
-    e = for_graph ? cudaSuccess : cudaEventSynchronize(meta_done_);
-    if (e != cudaSuccess) return cuda_fail(e, "waiting for the previous batch");
-    e = host_meta_.ensure(meta_bytes);
-    if (e != cudaSuccess) return cuda_fail(e, "allocating pinned descriptors");
+    if (!single) {
+        // the previous batch's descriptor copy must have left host_meta_
+        e = for_graph ? cudaSuccess : cudaEventSynchronize(meta_done_);
+        if (e != cudaSuccess) return cuda_fail(e, "waiting for the previous batch");
+        e = host_meta_.ensure(meta_bytes);
+        if (e != cudaSuccess) return cuda_fail(e, "allocating pinned descriptors");
+        std::memset(host_meta_.ptr, 0, meta_bytes);
+    }
     e = meta_.ensure(meta_bytes, st);
     if (e != cudaSuccess) return cuda_fail(e, "allocating device descriptors");
     char *h = static_cast<char *>(host_meta_.ptr);
     char *d = static_cast<char *>(meta_.ptr);
-    std::memset(h, 0, meta_bytes);
 
-    DevJob *hj = reinterpret_cast<DevJob *>(h + o_jobs);
+    DevJob one;
+    DevJob *hj = single ? &one : reinterpret_cast<DevJob *>(h + o_jobs);
     for (int i = 0; i < njobs; ++i) {
         const sarbp_job &j = jobs[i];
         DevJob &dj = hj[i];
@@ -536,40 +557,37 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         dj.wP = reinterpret_cast<float *>(sbase + lay[i].wP);
         dj.pulse = reinterpret_cast<double4 *>(sbase + lay[i].pulse);
         dj.sc = reinterpret_cast<JobScalars *>(sbase) + i;
+        dj.host_status = static_cast<int *>(status_pin_.ptr) + (size_t)i * kStatusWords;
         dj.nsplit = nsplit[i];
         dj.parts = nsplit[i] > 1 ? reinterpret_cast<float2 *>(sbase + lay[i].parts) : nullptr;
     }
-    RowItem *hr = reinterpret_cast<RowItem *>(h + o_rows);
-    std::vector<std::pair<int, size_t>> row_groups;  // (logN, first row)
-    size_t rpos = 0;
-    for (auto &kv : rows) {
-        row_groups.push_back({kv.first, rpos});
-        std::memcpy(hr + rpos, kv.second.data(), kv.second.size() * sizeof(RowItem));
-        rpos += kv.second.size();
-    }
-    std::memcpy(h + o_items, items.data(), items.size() * sizeof(WorkItem));
-    std::memcpy(h + o_tiles, tiles.data(), tiles.size() * sizeof(WorkItem));
-    std::memcpy(h + o_split, split.data(), split.size() * sizeof(int));
-
+    // The caller's inputs may still be on their way on the slabs' copy stream
+    // (and the descriptors of a batch go up behind them)
     cudaStream_t ms = (slabs && slabs->copy_stream) ? slabs->copy_stream : st;
-    e = cudaMemcpyAsync(d, h, meta_bytes, cudaMemcpyHostToDevice, ms);
-    if (e != cudaSuccess) return cuda_fail(e, "copying descriptors");
-    e = for_graph ? cudaSuccess : cudaEventRecord(meta_done_, ms);
+    if (!single) {
+        RowItem *hr = reinterpret_cast<RowItem *>(h + o_rows);
+        for (const RowGroup &g : row_groups)
+            std::memcpy(hr + g.first, rows[g.logN].data(), g.count * sizeof(RowItem));
+        std::memcpy(h + o_items, items.data(), items.size() * sizeof(WorkItem));
+        std::memcpy(h + o_tiles, tiles.data(), tiles.size() * sizeof(WorkItem));
+        e = cudaMemcpyAsync(d, h, meta_bytes, cudaMemcpyHostToDevice, ms);
+        if (e != cudaSuccess) return cuda_fail(e, "copying descriptors");
+    }
+    if (!for_graph && (!single || ms != st)) e = cudaEventRecord(meta_done_, ms);
     if (e == cudaSuccess && ms != st) e = cudaStreamWaitEvent(st, meta_done_, 0);
     if (e != cudaSuccess) return cuda_fail(e, "ordering the descriptor copy");
 
-    const DevJob *d_jobs = reinterpret_cast<const DevJob *>(d + o_jobs);
-    const RowItem *d_rows = reinterpret_cast<const RowItem *>(d + o_rows);
-    const WorkItem *d_items = reinterpret_cast<const WorkItem *>(d + o_items);
-    const WorkItem *d_tiles = split.empty() ? d_items : reinterpret_cast<const WorkItem *>(d + o_tiles);
-    const int ntile_items = split.empty() ? (int)items.size() : (int)tiles.size();
-    const int *d_split = reinterpret_cast<const int *>(d + o_split);
+    DevJob *d_jobs = reinterpret_cast<DevJob *>(d + o_jobs);
+    RowItem *d_rows = reinterpret_cast<RowItem *>(d + o_rows);
+    WorkItem *d_items = reinterpret_cast<WorkItem *>(d + o_items);
+    // (one job's items begin with part 0 of every tile)
+    const WorkItem *d_tiles = single || !any_split ? d_items : reinterpret_cast<const WorkItem *>(d + o_tiles);
     int *d_cnt = reinterpret_cast<int *>(d + o_cnt);
 
     // twiddle tables first (a one-time synchronous upload per N_fft; a
     // four-step N_fft also needs the tables of its two sub-lengths)
     for (size_t g = 0; g < row_groups.size(); ++g) {
-        const int l = row_groups[g].first;
+        const int l = row_groups[g].logN;
         const int need[3] = {l, l > kMaxLogNSmem ? l / 2 : l, l > kMaxLogNSmem ? l - l / 2 : l};
         for (int n : need) {
             float2 *tw = nullptr;
@@ -582,17 +600,23 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
     if (stage_events)
         for (int k = 0; k < DeviceInfo::kEvents; ++k) dev_->ev_recorded[k] = false;
     if ((e = rec(0)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
-    launch_prep(d_jobs, njobs, st);
+    if (single) {
+        e = launch_prep_single(one, SingleLists{d_jobs, d_items, (int)ntile_items, (int)nitems, d_rows,
+                                                (int)nrows_total, d_cnt, (int)(cnt_bytes / sizeof(int))}, st);
+        if (e != cudaSuccess) return cuda_fail(e, "set-up launch");
+    } else {
+        launch_prep(d_jobs, njobs, st);
+    }
     dev_->launches++;
     if ((e = rec(1)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
-    const bool slabbed = slabs && !items.empty() && prec[0] != SARBP_PREC_NAIVE;
+    const bool slabbed = slabs && nitems > 0 && prec[0] != SARBP_PREC_NAIVE;
     // Range compression beside the tile geometry: both read only the
     // set-up's tables, and the backprojection waits for both.  Each kernel
     // fills the SMs on its own, so they mostly fill each other's tails
     // (5.988 -> 5.979 ms per 2048^2 x 1999 step).  Not while the context
     // times its stages (each stage then runs alone), and not for row slabs
     // (their geometry already runs beside the backprojection).
-    const bool side = !rc_only && !slabbed && !items.empty() && !row_groups.empty() &&
+    const bool side = !rc_only && !slabbed && nitems > 0 && !row_groups.empty() &&
                       !(stage_events && dev_->timing && !for_graph);
     cudaStream_t rs = st;
     if (side) {
@@ -620,9 +644,8 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         ~Join() { now(); }
     } join{st, side_, side ? join_ : nullptr};
     for (size_t g = 0; g < row_groups.size(); ++g) {
-        const int logN = row_groups[g].first;
-        const size_t first = row_groups[g].second;
-        const size_t count = rows[logN].size();
+        const int logN = row_groups[g].logN;
+        const size_t first = row_groups[g].first, count = row_groups[g].count;
         float2 *work = work_bytes ? reinterpret_cast<float2 *>(sbase + work_off) : nullptr;
         e = range_compress_rows(dev_, logN, d_jobs, d_rows + first, (int)count, rc_only ? 0 : 1, work,
                                 rc_work_rows(logN), rs);
@@ -636,7 +659,7 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
                                 cudaMemcpyDeviceToDevice, st);
             if (e != cudaSuccess) return cuda_fail(e, "copying range profiles");
         }
-        if ((e = copy_status()) != cudaSuccess) return cuda_fail(e, "copying job status");
+        last_njobs_ = njobs;
         return SARBP_OK;
     }
     if (slabs && slabs->before_slabs && (e = slabs->before_slabs()) != cudaSuccess)
@@ -649,8 +672,8 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         const int tiles_x = (jobs[0].nu + L.tile_x - 1) / L.tile_x;
         if (bp_max_active_blocks(L) < 1) return fail(SARBP_ERR_CUDA, "backprojection kernel does not fit on an SM");
         for (int g = 0; g < slabs->nslabs; ++g) {
-            const size_t first = std::min(items.size(), (size_t)slabs->row0[g] * tiles_x);
-            const size_t last = std::min(items.size(), (size_t)std::max(slabs->row0[g], slabs->row0[g + 1]) * tiles_x);
+            const size_t first = std::min(nitems, (size_t)slabs->row0[g] * tiles_x);
+            const size_t last = std::min(nitems, (size_t)std::max(slabs->row0[g], slabs->row0[g + 1]) * tiles_x);
             cudaStream_t sg = (g & 1) ? slabs->aux : st;
             if ((g & 1) && (e = cudaStreamWaitEvent(sg, front_done_, 0)) != cudaSuccess)
                 return cuda_fail(e, "cudaStreamWaitEvent");
@@ -676,24 +699,25 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         for (int g = 1; g < slabs->nslabs; g += 2)
             if ((e = cudaStreamWaitEvent(st, slabs->done[g], 0)) != cudaSuccess)
                 return cuda_fail(e, "cudaStreamWaitEvent");
-        items.clear();  // formed above
+        nitems = 0;  // formed above
     }
-    if (!items.empty()) {
-        e = launch_tile_setup(d_jobs, d_tiles, ntile_items, L.tile_x * L.tile_y, st);
+    if (nitems > 0) {
+        e = launch_tile_setup(d_jobs, d_tiles, (int)ntile_items, L.tile_x * L.tile_y, st);
         if (e != cudaSuccess) return cuda_fail(e, "tile geometry launch");
         dev_->launches += 1;
     }
     if ((e = join.now()) != cudaSuccess) return cuda_fail(e, "ordering range compression");
     if (!slabbed && (e = rec(3)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
-    if (!items.empty()) {
+    if (nitems > 0) {
         if (L.persistent) {
             const int occ = bp_max_active_blocks(L);
             if (occ < 1) return fail(SARBP_ERR_CUDA, "backprojection kernel does not fit on an SM");
-            L.grid = std::min<long long>((long long)occ * dev_->num_sms, (long long)items.size());
-            // sorted longest first: equal when the ends differ by a pulse at
-            // most (parts of one job).  Uneven lists: even shares of pulses
-            // over the last three rounds of the longest item
-            const int longest = item_pulses(items.front()), shortest = item_pulses(items.back());
+            L.grid = std::min<long long>((long long)occ * dev_->num_sms, (long long)nitems);
+            // one job's items, or ones sorted longest first whose ends differ by
+            // a pulse at most, are equal (parts of one job differ by a pulse).
+            // Uneven lists: even shares of pulses over the last three rounds of
+            // the longest item
+            const int longest = single ? 0 : item_pulses(items.front()), shortest = single ? 0 : item_pulses(items.back());
             if (longest - shortest <= 1) {
                 L.deal.how = kDealItems;
             } else {
@@ -707,15 +731,8 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
                 if (total < (1ll << 31)) L.deal = BpDeal{kDealPulses, (int)zone, total};
             }
         }
-        e = launch_backproject(L, d_jobs, d_items, (int)items.size(), d_cnt, st);
+        e = launch_backproject(L, d_jobs, d_items, (int)nitems, d_cnt, st);
         if (e != cudaSuccess) return cuda_fail(e, "backprojection launch");
-        dev_->launches++;
-    }
-    if (!split.empty()) {
-        long long px = 0;
-        for (int i : split) px = std::max(px, (long long)jobs[i].nu * jobs[i].nv);
-        e = launch_combine_parts(d_jobs, d_split, (int)split.size(), px, dev_->num_sms, st);
-        if (e != cudaSuccess) return cuda_fail(e, "pulse-part combine launch");
         dev_->launches++;
     }
     for (int i : naive) {
@@ -739,7 +756,7 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         dev_->launches++;
         if ((e = rec(5)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
     }
-    if ((e = copy_status()) != cudaSuccess) return cuda_fail(e, "copying job status");
+    last_njobs_ = njobs;
     return SARBP_OK;
 }
 
@@ -747,9 +764,10 @@ int Runner::check_status(cudaStream_t st) {
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "synchronising the stream");
     if (last_njobs_ == 0 || !status_pin_.ptr) return SARBP_OK;
-    const JobScalars *sc = static_cast<const JobScalars *>(status_pin_.ptr);
+    const volatile int *words = static_cast<const int *>(status_pin_.ptr);
     for (int i = 0; i < last_njobs_; ++i) {
-        const int s = sc[i].status;
+        int s = 0;
+        for (int k = 0; k < kStatusWords; ++k) s |= words[i * kStatusWords + k] ? 1 << k : 0;
         if (s & kStatusNonFinite)
             return fail(SARBP_ERR_GEOMETRY, "job " + std::to_string(i) +
                                                 ": non-finite pixel or antenna position (those "

@@ -148,7 +148,7 @@ private:
     cudaStream_t side_ = nullptr;
     cudaEvent_t fork_ = nullptr, join_ = nullptr;
     int last_njobs_ = 0;
-    PinnedBuffer status_pin_;          // JobScalars of the last batch, copied behind it
+    PinnedBuffer status_pin_;          // kStatusWords per job, set by the kernels
     cudaMemPool_t pool_ = nullptr;
 };
 

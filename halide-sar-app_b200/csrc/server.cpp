@@ -635,12 +635,8 @@ int sarbp_server_register(sarbp_server *s, const sarbp_job *host_aperture, long 
     dj.pulse = reinterpret_cast<double4 *>(tb + o_pulse);
     DevJob *d_job = reinterpret_cast<DevJob *>(tb + o_job);
     auto *rows = reinterpret_cast<RowItem *>(tb + o_rows);
-    if (e == cudaSuccess) e = launch_store_job(dj, d_job, st);
-    if (e == cudaSuccess) {
-        launch_prep(d_job, 1, st);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = launch_fill_items(nullptr, 0, rows, (int)P, st);
+    if (e == cudaSuccess)
+        e = launch_prep_single(dj, SingleLists{d_job, nullptr, 0, 0, rows, (int)P, nullptr, 0}, st);
     if (e == cudaSuccess)
         e = range_compress_rows(&s->ctx->dev, dj.logN, d_job, rows, (int)P, 1, reinterpret_cast<float2 *>(tb + o_work),
                                 rc_work_rows(dj.logN), st);
@@ -653,7 +649,7 @@ int sarbp_server_register(sarbp_server *s, const sarbp_job *host_aperture, long 
         uncharge(res_bytes + tmp_bytes);
         return cuda_fail(e, "registering an aperture: upload and range compression");
     }
-    s->ctx->dev.launches += 4;
+    s->ctx->dev.launches += 2;
     s->h2d_bytes += (long long)(P * S * 8 + (h.k_r ? S * 4 : 0) + (h.k_r64 ? S * 8 : 0) + (h.pos ? P * 12 : 0) +
                                 (h.pos64 ? P * 24 : 0));
     s->rc_pulses += (long long)P;

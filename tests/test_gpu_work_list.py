@@ -73,3 +73,19 @@ def test_uneven_list_equals_each_job_alone(ctx, torch, precise):
     jobs[0].run(ctx, jobs=[j.job for j in jobs])
     for j, (img, u8) in zip(jobs, alone):
         assert np.array_equal(img, j.out.cpu().numpy()) and np.array_equal(u8, j.u8.cpu().numpy())
+
+
+# the fewest and the most parts, odd counts, parts of one pulse
+@pytest.mark.parametrize("parts,P", [(2, 65), (5, 97), (16, 16), (16, 200)])
+def test_parts_summed_by_the_last_item(ctx, torch, parts, P):
+    """The same bits whichever CTA completes a tile, alone and in a batch; the
+    sum over parts differs from one item per tile by f32 rounding only (P
+    terms: about sqrt(P) 2^-24 of the sum, well below 1e-5)."""
+    a, b = _Job(torch, 200, 130, P, seed=P), _Job(torch, 90, 300, P + 3, seed=P + 1)
+    whole = a.run(ctx, pulse_parts=1)[0]
+    first = a.run(ctx, pulse_parts=parts)
+    assert np.linalg.norm(first[0] - whole) < 1e-5 * np.linalg.norm(whole)
+    for _ in range(10):
+        a.out.fill_(-7.0)
+        again = a.run(ctx, jobs=[a.job, b.job], pulse_parts=parts)
+        assert np.array_equal(first[0], again[0]) and np.array_equal(first[1], again[1])
