@@ -542,10 +542,7 @@ __device__ __forceinline__ void producer_loop(const DevJob *__restrict__ jobs,
             const TileInfo &ti = jb.tiles[wi.tile];
             sh = tile_shape(ti, pe - pb, stage_cap, cmax);
             flags = (ti.planar ? kChunkPlanar : 0) | (ti.wide ? kChunkWide : 0);
-            if (persistent && lane == 0) {
-                if (n == 0) claims.start(pe - pb);
-                else if (deal.how != kDealNone) claims.account(pe - pb);
-            }
+            if (n > 0 && deal.how != kDealNone && lane == 0) claims.account(pe - pb);
         }
         bool ok = true;
         // an item without chunks (tile too wide) and the end take one empty turn
@@ -569,6 +566,8 @@ __device__ __forceinline__ void producer_loop(const DevJob *__restrict__ jobs,
                                               (c == turns - 1 ? kChunkLast : 0));
             __syncwarp();
             bar_arrive(kBarFull0 + b);
+            // after the first chunk: its atomics would hold it back
+            if (g == 0 && lane == 0) claims.start(pe - pb);
         }
         if (!more) break;
         if (!ok && lane == 0) report_status(jb, kStatusTimeout);
@@ -578,24 +577,39 @@ __device__ __forceinline__ void producer_loop(const DevJob *__restrict__ jobs,
     if (g >= 2) bar_sync(kBarEmpty0 + (g & 1));
 }
 
+// The pixels of a consumer thread: n of them (k = 0 .. n - 1, at most PPT)
+// inside the image, `step` apart from pixel (ix, iy).  Lanes run along x, or
+// along y on transposed tiles (square tiles whose range bins step faster
+// along x than along y, so that neighbouring lanes read neighbouring or equal
+// window entries).  The set-up and the epilogue of an item run once per tile
+// from a cold instruction cache, so they are kept short.
+template <int TX, int TY>
+struct PixelRun {
+    static constexpr int ROWS = kConsumers / TX;
+    int ix, iy, n;
+    bool tr;
+    __device__ __forceinline__ explicit PixelRun(const ItemCtx &it) {
+        const int lx = threadIdx.x % TX, ly = threadIdx.x / TX;
+        tr = TX == TY && (it.flags & kItemTransposed);
+        ix = it.tx0 + (tr ? ly : lx);
+        iy = it.ty0 + (tr ? lx : ly);
+        const int along = tr ? it.nu - ix : it.nv - iy;
+        n = (tr ? iy < it.nv : ix < it.nu) ? (along + ROWS - 1) / ROWS : 0;
+        if (n <= 0) {  // none: the tile's first pixel stands in for loads
+            ix = it.tx0;
+            iy = it.ty0;
+        }
+    }
+    __device__ __forceinline__ long long first(const ItemCtx &it) const { return (long long)iy * it.nu + ix; }
+    __device__ __forceinline__ long long step(const ItemCtx &it) const { return tr ? ROWS : (long long)ROWS * it.nu; }
+    // k, or 0 outside the image
+    __device__ __forceinline__ int in(int k) const { return k < n ? k : 0; }
+};
+
 template <int TX, int TY, bool PRE>
 __device__ __forceinline__ void consumer_loop(int stage_cap, int cmax, const TileSmem &sm) {
     constexpr int PPT = TX * TY / kConsumers;
-    constexpr int ROWS = kConsumers / TX;
     const int tid = threadIdx.x;
-    // pixel k of this thread: lanes run along x, or along y on transposed
-    // tiles (square tiles whose range bins step faster along x than along y,
-    // so that neighbouring lanes read neighbouring or equal window entries)
-    auto pixel_of = [&](const ItemCtx &it, int k, int &ix, int &iy) {
-        const int lx = tid % TX, ly = tid / TX;
-        if (TX == TY && (it.flags & kItemTransposed)) {
-            ix = it.tx0 + ly + k * ROWS;
-            iy = it.ty0 + lx;
-        } else {
-            ix = it.tx0 + lx;
-            iy = it.ty0 + ly + k * ROWS;
-        }
-    };
     const uint32_t stage_base = smem_u32(sm.stage) - kMagicOff;
     constexpr int NP = PPT / 2;
     // pixel pairs (2j, 2j + 1) for the f32x2 arithmetic
@@ -609,53 +623,56 @@ __device__ __forceinline__ void consumer_loop(int stage_cap, int cmax, const Til
             // ---- pixel offsets from the tile centre, in radians ----
             const ItemCtx &it = sm.ctx[ch.x];
             ilk = it.ilk;
+            const PixelRun<TX, TY> px(it);
             double x[PPT], y[PPT], z[PPT];
-            bool in[PPT];
-            // all positions are loaded before the first is used (pixels
-            // outside the image read the edge's and are dropped below)
+            // all positions are loaded before the first is used
+            if (it.r) {
+                const long long npix = (long long)it.nu * it.nv, step = px.step(it);
+                const double *r = it.r + px.first(it);
 #pragma unroll
-            for (int k = 0; k < PPT; ++k) {
-                int ix, iy;
-                pixel_of(it, k, ix, iy);
-                in[k] = ix < it.nu && iy < it.nv;
-                ix = min(ix, it.nu - 1);
-                iy = min(iy, it.nv - 1);
-                if (it.r) {
-                    const long long npix = (long long)it.nu * it.nv;
-                    const long long pix = (long long)iy * it.nu + ix;
-                    x[k] = it.r[pix];
-                    y[k] = it.r[npix + pix];
-                    z[k] = it.r[2 * npix + pix];
-                } else {
+                for (int k = 0; k < PPT; ++k) {
+                    const double *q = r + px.in(k) * step;
+                    x[k] = q[0];
+                    y[k] = q[npix];
+                    z[k] = q[2 * npix];
+                }
+            } else {
+                const double *u = it.u + px.ix, *v = it.v + px.iy;
+                double uu[PPT], vv[PPT];
+#pragma unroll
+                for (int k = 0; k < PPT; ++k) {
+                    const int d = px.in(k) * px.ROWS;
+                    uu[k] = u[px.tr ? d : 0];
+                    vv[k] = v[px.tr ? 0 : d];
+                }
+#pragma unroll
+                for (int k = 0; k < PPT; ++k) {
                     // img_plane.cpp:92-102: (0 + u_hat*u) + v_hat*v
-                    const double uu = it.u[ix], vv = it.v[iy];
-                    x[k] = __dadd_rn(__dmul_rn(it.uh[0], uu), __dmul_rn(it.vh[0], vv));
-                    y[k] = __dadd_rn(__dmul_rn(it.uh[1], uu), __dmul_rn(it.vh[1], vv));
-                    z[k] = __dadd_rn(__dmul_rn(it.uh[2], uu), __dmul_rn(it.vh[2], vv));
+                    x[k] = __dadd_rn(__dmul_rn(it.uh[0], uu[k]), __dmul_rn(it.vh[0], vv[k]));
+                    y[k] = __dadd_rn(__dmul_rn(it.uh[1], uu[k]), __dmul_rn(it.vh[1], vv[k]));
+                    z[k] = __dadd_rn(__dmul_rn(it.uh[2], uu[k]), __dmul_rn(it.vh[2], vv[k]));
                 }
             }
-            float dx[PPT], dy[PPT], dz[PPT], nd2[PPT], s0[PPT];
 #pragma unroll
             for (int k = 0; k < PPT; ++k) {
-                dx[k] = dy[k] = dz[k] = nd2[k] = s0[k] = 0.0f;
-                if (in[k] && isfinite(x[k]) && isfinite(y[k]) && isfinite(z[k])) {
+                float dx = 0.0f, dy = 0.0f, dz = 0.0f, nd2 = 0.0f, s0 = 0.0f;
+                if (k < px.n && isfinite(x[k]) && isfinite(y[k]) && isfinite(z[k])) {
                     // the same f32 offsets the tile set-up measured rho on
-                    dx[k] = it.kcf * (float)(x[k] - it.rc[0]);
-                    dy[k] = it.kcf * (float)(y[k] - it.rc[1]);
-                    dz[k] = it.kcf * (float)(z[k] - it.rc[2]);
-                    nd2[k] = -fmaf(dx[k], dx[k], fmaf(dy[k], dy[k], dz[k] * dz[k]));
-                    s0[k] = fmaf(it.w0[2], dz[k], fmaf(it.w0[1], dy[k], it.w0[0] * dx[k]));
+                    dx = it.kcf * (float)(x[k] - it.rc[0]);
+                    dy = it.kcf * (float)(y[k] - it.rc[1]);
+                    dz = it.kcf * (float)(z[k] - it.rc[2]);
+                    nd2 = -fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                    s0 = fmaf(it.w0[2], dz, fmaf(it.w0[1], dy, it.w0[0] * dx));
                 }
+                float2 &DX = dxp[k >> 1], &DY = dyp[k >> 1], &DZ = dzp[k >> 1], &ND2 = nd2p[k >> 1], &S0 = s0p[k >> 1];
+                ((k & 1) ? DX.y : DX.x) = dx;
+                ((k & 1) ? DY.y : DY.x) = dy;
+                ((k & 1) ? DZ.y : DZ.x) = dz;
+                ((k & 1) ? ND2.y : ND2.x) = nd2;
+                ((k & 1) ? S0.y : S0.x) = s0;
             }
 #pragma unroll
-            for (int j = 0; j < NP; ++j) {
-                dxp[j] = make_float2(dx[2 * j], dx[2 * j + 1]);
-                dyp[j] = make_float2(dy[2 * j], dy[2 * j + 1]);
-                dzp[j] = make_float2(dz[2 * j], dz[2 * j + 1]);
-                nd2p[j] = make_float2(nd2[2 * j], nd2[2 * j + 1]);
-                s0p[j] = make_float2(s0[2 * j], s0[2 * j + 1]);
-                arp[j] = aip[j] = make_float2(0.0f, 0.0f);
-            }
+            for (int j = 0; j < NP; ++j) arp[j] = aip[j] = make_float2(0.0f, 0.0f);
         }
         {
             const float2 ILK = make_float2(ilk, ilk);
@@ -679,54 +696,54 @@ __device__ __forceinline__ void consumer_loop(int stage_cap, int cmax, const Til
         // goes on with the slices' sum, a pulse chunk adds its sums to the
         // partial image instead; loads before the first store ----
         const ItemCtx &it = sm.ctx[done.x];
+        const PixelRun<TX, TY> px(it);
+        const long long at = px.first(it), step = px.step(it);
         float2 sum[PPT], in[PPT];  // the item's sums; final phases, or the partial image so far
-        long long at[PPT];         // pixel, -1 outside the image
+        const float2 *src = ((it.flags & kItemAcc) ? it.sums : it.fin) + at;
 #pragma unroll
-        for (int k = 0; k < PPT; ++k) {
-            int ix, iy;
-            pixel_of(it, k, ix, iy);
-            at[k] = ix < it.nu && iy < it.nv ? (long long)iy * it.nu + ix : -1;
+        for (int k = 0; k < PPT; ++k) in[k] = src[px.in(k) * step];
+#pragma unroll
+        for (int k = 0; k < PPT; ++k)
             sum[k] = make_float2((k & 1) ? arp[k >> 1].y : arp[k >> 1].x, (k & 1) ? aip[k >> 1].y : aip[k >> 1].x);
-        }
-        if (it.flags & kItemPart) {
+        if (it.flags & (kItemPart | kItemAcc)) {
+            float2 *dst = it.sums + at;
+            const bool acc = (it.flags & kItemAcc) != 0;
 #pragma unroll
             for (int k = 0; k < PPT; ++k)
-                if (at[k] >= 0) it.sums[at[k]] = sum[k];
+                if (k < px.n) dst[k * step] = acc ? make_float2(in[k].x + sum[k].x, in[k].y + sum[k].y) : sum[k];
+            if (acc) continue;
             __threadfence();  // the slice before the count
             asm volatile("bar.sync %0, %1;" ::"r"(kBarConsumers), "r"(kConsumers) : "memory");
-            if (tid == 0) *sm.s_last = atomicAdd(it.done, 1) == it.nsplit - 1;
+            if (tid == 0) {
+                *sm.s_last = atomicAdd(it.done, 1) == it.nsplit - 1;
+                __threadfence();  // the count before the other slices
+            }
             asm volatile("bar.sync %0, %1;" ::"r"(kBarConsumers), "r"(kConsumers) : "memory");
             if (!*sm.s_last) continue;
-            __threadfence();
+            const float2 *part = it.parts + at;
             const long long npix = (long long)it.nu * it.nv;
 #pragma unroll
-            for (int k = 0; k < PPT; ++k)
-                if (at[k] >= 0) sum[k] = __ldcg(it.parts + at[k]);
-#pragma unroll 4
-            for (int p = 1; p < it.nsplit; ++p)
+            for (int k = 0; k < PPT; ++k) sum[k] = __ldcg(part + px.in(k) * step);
+#pragma unroll 1
+            for (int p = 1; p < it.nsplit; ++p) {
+                part += npix;
 #pragma unroll
-                for (int k = 0; k < PPT; ++k)
-                    if (at[k] >= 0) {
-                        const float2 s = __ldcg(it.parts + p * npix + at[k]);
-                        sum[k].x += s.x;
-                        sum[k].y += s.y;
-                    }
+                for (int k = 0; k < PPT; ++k) {
+                    const float2 s = __ldcg(part + px.in(k) * step);
+                    sum[k].x += s.x;
+                    sum[k].y += s.y;
+                }
+            }
         }
-        const bool acc = (it.flags & kItemAcc) != 0;
-#pragma unroll
-        for (int k = 0; k < PPT; ++k) in[k] = at[k] >= 0 ? (acc ? it.sums : it.fin)[at[k]] : make_float2(0.0f, 0.0f);
+        double2 *out = it.out + ((long long)(it.nv - 1 - px.iy) * it.nu + px.ix);
+        const long long ostep = px.tr ? step : -step;  // rows are flipped
         double zmax = 0.0;
 #pragma unroll
         for (int k = 0; k < PPT; ++k) {
-            if (at[k] < 0) continue;
-            if (acc) {
-                it.sums[at[k]] = make_float2(in[k].x + sum[k].x, in[k].y + sum[k].y);
-            } else {
-                const double zr = (double)fmaf(sum[k].x, in[k].x, -sum[k].y * in[k].y);
-                const double zi = (double)fmaf(sum[k].x, in[k].y, sum[k].y * in[k].x);
-                int ix, iy;
-                pixel_of(it, k, ix, iy);
-                it.out[(long long)(it.nv - 1 - iy) * it.nu + ix] = make_double2(zr, zi);
+            const double zr = (double)fmaf(sum[k].x, in[k].x, -sum[k].y * in[k].y);
+            const double zi = (double)fmaf(sum[k].x, in[k].y, sum[k].y * in[k].x);
+            if (k < px.n) {
+                out[k * ostep] = make_double2(zr, zi);
                 if (it.flags & kItemMax) zmax = fmax(zmax, sqrt(zr * zr + zi * zi));
             }
         }
