@@ -341,7 +341,7 @@ int sarbp_accum_finalize(sarbp_accum *acc) {
     cudaError_t e = launch_finalize(f, acc->npix, acc->ctx->dev.num_sms, s);
     int nl = 1;
     if (e == cudaSuccess && acc->job.out_u8) {
-        e = launch_batch_u8(acc->d_job(), 1, acc->npix, s);
+        e = launch_batch_u8(acc->d_job(), 1, u8_chunks(acc->npix), s);
         ++nl;
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(acc->status_pin.ptr, sc, sizeof(JobScalars), cudaMemcpyDeviceToHost, s);

@@ -408,14 +408,10 @@ int sarbp_img_output_to_dB_device(sarbp_ctx *ctx, const double *img, int nu, int
     int rc = set_device(ctx);
     if (rc) return rc;
     if (!img || !dB || nu < 1 || nv < 1) return fail(SARBP_ERR_INVALID, "bad dB arguments");
-    cudaError_t e = ctx->out_aux.ensure(256, ctx->stream);
+    cudaError_t e = ctx->out_aux.ensure(kMaxParts * sizeof(double), ctx->stream);
     if (e != cudaSuccess) return cuda_fail(e, "allocating");
-    auto *m = static_cast<unsigned long long *>(ctx->out_aux.ptr);
-    e = cudaMemsetAsync(m, 0, sizeof(unsigned long long), ctx->stream);
-    if (e == cudaSuccess) e = launch_maxabs(reinterpret_cast<const double2 *>(img), (long long)nu * nv, m, ctx->stream);
-    if (e == cudaSuccess)
-        e = launch_db_u8(reinterpret_cast<const double2 *>(img), (long long)nu * nv, m, dB, nullptr, 0, 1,
-                         ctx->stream);
+    e = launch_db(reinterpret_cast<const double2 *>(img), (long long)nu * nv, static_cast<double *>(ctx->out_aux.ptr),
+                  dB, ctx->stream);
     if (e != cudaSuccess) return cuda_fail(e, "dB launch");
     ctx->dev.launches += 2;
     return SARBP_OK;
@@ -439,14 +435,10 @@ int sarbp_img_output_u8_from_img_device(sarbp_ctx *ctx, const double *img, int n
     if (rc) return rc;
     if (!img || !out || nu < 1 || nv < 1) return fail(SARBP_ERR_INVALID, "bad u8 arguments");
     if (!(dB_min < dB_max)) return fail(SARBP_ERR_INVALID, "Constraint failed: dB_min < dB_max");
-    cudaError_t e = ctx->out_aux.ensure(256, ctx->stream);
+    cudaError_t e = ctx->out_aux.ensure(kMaxParts * sizeof(double), ctx->stream);
     if (e != cudaSuccess) return cuda_fail(e, "allocating");
-    auto *m = static_cast<unsigned long long *>(ctx->out_aux.ptr);
-    const long long n = (long long)nu * nv;
-    e = cudaMemsetAsync(m, 0, sizeof(unsigned long long), ctx->stream);
-    if (e == cudaSuccess) e = launch_maxabs(reinterpret_cast<const double2 *>(img), n, m, ctx->stream);
-    if (e == cudaSuccess)
-        e = launch_img_u8(reinterpret_cast<const double2 *>(img), n, m, out, dB_min, dB_max, ctx->stream);
+    e = launch_img_u8(reinterpret_cast<const double2 *>(img), (long long)nu * nv,
+                      static_cast<double *>(ctx->out_aux.ptr), out, dB_min, dB_max, ctx->stream);
     if (e != cudaSuccess) return cuda_fail(e, "u8 launch");
     ctx->dev.launches += 2;
     return SARBP_OK;

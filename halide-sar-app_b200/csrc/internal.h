@@ -15,6 +15,7 @@ namespace sarbp {
 constexpr int kMaxTaylorTerms = 64;  // n_bar - 1 <= 64  (S_L up to ~150 dB)
 constexpr int kMinLogN = 4;          // N_fft in [16, 131072]
 constexpr int kMaxLogN = 17;
+constexpr int kU8Chunk = 1024;       // pixels of one chunk of the batch's u8 kernel
 constexpr int kMaxLogNSmem = 14;     // up to here one CTA holds a whole row
 
 // status bits written by kernels into JobScalars::status
@@ -107,6 +108,7 @@ struct DevJob {
     double2 *out;         // [nv][nu]
     uint8_t *out_u8;      // [nv][nu] or null
     double dB_min, dB_max;
+    long long u8_chunk0;  // the job's first chunk of the u8 kernel (jobs with out_u8)
     // pulse-chunked jobs: the descriptor of one chunk has P = the chunk's
     // pulses, phs its phase-history rows in order (no fftshift rotation:
     // wP and pulse are the chunk's gathered window and pulse table), and
@@ -139,6 +141,9 @@ __host__ __device__ inline void part_range(int P, int nsplit, int part, int &p0,
     p0 = (int)((long long)part * P / nsplit);
     p1 = (int)((long long)(part + 1) * P / nsplit);
 }
+
+// Chunks of the u8 kernel in an image of npix pixels.
+inline long long u8_chunks(long long npix) { return (npix + kU8Chunk - 1) / kU8Chunk; }
 
 #ifdef __CUDACC__
 // Sets status bit `bit` of a job.

@@ -110,15 +110,16 @@ cudaError_t launch_resize(const ResizePlan &p, const void *in, void *out, void *
 cudaError_t measure_peaks(int num_sms, cudaStream_t st, double *ffma_per_s, double *mufu_per_s);
 
 // output.cu
-cudaError_t launch_maxabs(const double2 *img, long long n, unsigned long long *d_max, cudaStream_t st);
-cudaError_t launch_db_u8(const double2 *img, long long n, const unsigned long long *d_max,
-                         double *dB, uint8_t *u8, double dB_min, double dB_max, cudaStream_t st);
+// dB image and u8 image of a complex image, each a pass for max |z|^2 and a pass
+// over the pixels (two launches); part: kMaxParts doubles of scratch
+constexpr int kMaxParts = 4096;
+cudaError_t launch_db(const double2 *img, long long n, double *part, double *dB, cudaStream_t st);
+cudaError_t launch_img_u8(const double2 *img, long long n, double *part, uint8_t *u8, double lo, double hi,
+                          cudaStream_t st);
 cudaError_t launch_u8_from_db(const double *dB, long long n, double dB_min, double dB_max,
                               uint8_t *u8, cudaStream_t st);
-// u8 image straight from a complex image and its max|z| (no f64 dB image)
-cudaError_t launch_img_u8(const double2 *img, long long n, const unsigned long long *d_max, uint8_t *u8,
-                          double lo, double hi, cudaStream_t st);
-// u8 images of every job of a batch that asked for one (uses DevJob::maxabs)
-cudaError_t launch_batch_u8(const DevJob *d_jobs, int njobs, long long max_pixels, cudaStream_t st);
+// u8 images of every job of a batch that asked for one (uses JobScalars::maxabs):
+// `chunks` of kU8Chunk pixels, job i's from DevJob::u8_chunk0 on
+cudaError_t launch_batch_u8(const DevJob *d_jobs, int njobs, long long chunks, cudaStream_t st);
 
 }  // namespace sarbp

@@ -258,7 +258,7 @@ extern "C" int sarbp_backprojection_noalloc(const sarbp_job *job, void *cuda_str
     L.grid = (int)std::min<long long>((long long)occ * num_sms, (long long)nitems);
     L.deal.how = kDealItems;  // one job: its parts differ by a pulse at most
     e = launch_backproject(L, d_job, d_items, (int)nitems, d_cnt, st);
-    if (e == cudaSuccess && j.out_u8) e = launch_batch_u8(d_job, 1, (long long)j.nu * j.nv, st);
+    if (e == cudaSuccess && j.out_u8) e = launch_batch_u8(d_job, 1, u8_chunks((long long)j.nu * j.nv), st);
     if (e == cudaSuccess && status) {
         status_kernel<<<1, 1, 0, st>>>(dj.sc, status);
         e = cudaGetLastError();

@@ -5,10 +5,11 @@
 //         log(Expr(10)) has an integer argument, so Halide takes it in f32)
 //   u8  = trunc(clamp((clamp(dB, lo, hi) - lo) / (hi - lo) * 255, 0, 255))
 //                                              (img_output.cpp:48-51, signal.h:55-57)
-// All HBM-bound; the fused form reads the complex image once and writes the
-// u8 (and optionally the f64 dB) image, using the max|z| that the
-// backprojection epilogue already reduced.
+// HBM-bound but for the f64 logarithm of the dB image; the u8 form reads the
+// complex image once and writes the u8 image, using the max|z| that the
+// backprojection epilogue already reduced where there is one.
 #include <algorithm>
+#include <cfloat>
 #include <cstdint>
 
 #include "internal.h"
@@ -31,9 +32,11 @@ __device__ __forceinline__ uint8_t to_u8(double v, double lo, double hi) {
 // u8 of one pixel.  The value is decided in f32 (|z|^2 rounded to f32, the
 // accurate logf), whose error is far below 1e-4 of a grey level for display
 // ranges of 0.1 dB and wider; a pixel whose f32 level lands within that
-// margin of an integer, of the clamps, or is not finite, is recomputed with
-// the reference's f64 formula.  Only the f64 path runs where dB itself is
-// written.
+// margin of an integer or of the clamps, or whose f32 values are not normal
+// numbers, is recomputed with the reference's f64 formula.  Pixels clearly
+// below dB_min or above dB_max are decided in f32 as well: in a scene of a few
+// bright points that is most of them (12 jobs of 256^2 to 1024^2 pixels, -40
+// dB: 81 us with those in f64, 31 us without).
 struct U8Scale {
     double m, lo, hi;
     float inv_m2, k, q0, eps;  // q = k ln(|z|^2 / m^2) + q0 (grey levels)
@@ -49,14 +52,20 @@ __device__ __forceinline__ U8Scale u8_scale(double m, double lo, double hi) {
     u.k = (float)(5.0 / kLn10F32 * g);                // 10 log10(a/m) = 5 ln(a^2/m^2) / ln 10
     u.q0 = (float)(-lo * g);
     u.eps = (float)(2e-5 * g + 1e-4);
+    if (!(u.inv_m2 >= FLT_MIN && u.inv_m2 <= FLT_MAX)) u.eps = INFINITY;  // every pixel in f64
     return u;
 }
 
 __device__ __forceinline__ uint8_t u8_of(double2 z, const U8Scale &u) {
     const double a2 = z.x * z.x + z.y * z.y;
-    const float q = fmaf(u.k, logf((float)a2 * u.inv_m2), u.q0);
+    const float a = (float)a2;
+    const float q = fmaf(u.k, logf(a * u.inv_m2), u.q0);
     const float f = q - floorf(q);
-    if (q > u.eps && q < 255.0f - u.eps && f > u.eps && f < 1.0f - u.eps) return (uint8_t)q;
+    if (a >= FLT_MIN && a <= FLT_MAX) {  // (an f32 overflow or underflow says nothing)
+        if (q > u.eps && q < 255.0f - u.eps && f > u.eps && f < 1.0f - u.eps) return (uint8_t)q;
+        if (q < -u.eps) return 0;
+        if (q > 255.0f + u.eps) return 255;
+    }
     return to_u8(10.0 * (log(sqrt(a2) / u.m) / kLn10F32), u.lo, u.hi);
 }
 
@@ -64,8 +73,10 @@ __device__ __forceinline__ uint8_t u8_of(double2 z, const U8Scale &u) {
 // warp's loads stay contiguous), the maximum taken on |z|^2 and one square
 // root at the end -- the same value, as the square root is monotonic and
 // correctly rounded.
-__global__ void maxabs_kernel(const double2 *__restrict__ img, long long n,
-                              unsigned long long *__restrict__ out) {
+// One maximum of |z|^2 per CTA; the kernel that uses it takes the maximum of
+// those (image_max2), so nothing has to be cleared ahead of the pass.
+__global__ void __launch_bounds__(256) max2_kernel(const double2 *__restrict__ img, long long n,
+                                                   double *__restrict__ part) {
     double m2 = 0.0;
     const long long stride = (long long)gridDim.x * blockDim.x;
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -80,33 +91,71 @@ __global__ void maxabs_kernel(const double2 *__restrict__ img, long long n,
         const double2 z = img[i];
         m2 = fmax(m2, z.x * z.x + z.y * z.y);
     }
-    double m = sqrt(m2);
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    __shared__ double s[32];
-    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = m;
+    for (int o = 16; o > 0; o >>= 1) m2 = fmax(m2, __shfl_xor_sync(0xffffffffu, m2, o));
+    __shared__ double s[8];
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = m2;
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, s[w]);
-        atomicMax(out, (unsigned long long)__double_as_longlong(m));
+        for (int w = 1; w < 8; ++w) m2 = fmax(m2, s[w]);
+        part[blockIdx.x] = m2;
     }
 }
 
-__global__ void db_u8_kernel(const double2 *__restrict__ img, long long n,
-                             const unsigned long long *__restrict__ maxbits, double *__restrict__ dB,
-                             uint8_t *__restrict__ u8, double lo, double hi) {
-    const double m = __longlong_as_double((long long)*maxbits);
-    const U8Scale us = u8_scale(m, lo, hi);
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        const double2 z = img[i];
-        if (!dB) {
-            u8[i] = u8_of(z, us);
-            continue;
+// max |z|^2 of the image from its partial maxima, in every thread of a CTA of 256
+__device__ __forceinline__ double image_max2(const double *__restrict__ part, int nparts) {
+    double m2 = 0.0;
+    for (int i = threadIdx.x; i < nparts; i += 256) m2 = fmax(m2, part[i]);
+    for (int o = 16; o > 0; o >>= 1) m2 = fmax(m2, __shfl_xor_sync(0xffffffffu, m2, o));
+    __shared__ double s[8];
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = m2;
+    __syncthreads();
+    for (int w = 0; w < 8; ++w) m2 = fmax(m2, s[w]);
+    return m2;
+}
+
+// dB of one pixel.  The reference's 10 (log(|z| / m) / ln 10) takes a square
+// root and two divisions besides the logarithm, and the f64 pipe is what
+// bounds the kernel; here it is 5 / ln 10 times the logarithm of
+// |z|^2 * (1 / m^2), whose three roundings weigh as much with the factor 5 as
+// the reference's with 10 (same error against 64-bit values, 1.1e-16).  The
+// maximum itself stays at exactly 0 and nothing above it; a maximum whose
+// square is not an ordinary number takes the reference's formula.
+// 2048^2: 22 us, 31 before.
+struct DbScale {
+    double m2, inv, m;
+    bool plain;
+};
+__device__ __forceinline__ DbScale db_scale(double m2) {
+    return DbScale{m2, 1.0 / m2, sqrt(m2), m2 > 1e-290 && m2 < 1e290};
+}
+__device__ __forceinline__ double db_of(double2 z, const DbScale &s) {
+    const double a2 = z.x * z.x + z.y * z.y;
+    if (!s.plain) return 10.0 * (log(sqrt(a2) / s.m) / kLn10F32);
+    const double q = a2 == s.m2 ? 1.0 : a2 * s.inv;
+    return fmin(5.0 / kLn10F32 * log(q), q == q ? 0.0 : q);
+}
+
+// Two neighbouring pixels a thread and step: 32 B in, 16 B out where dB is
+// 16-byte aligned.
+__global__ void __launch_bounds__(256) db_kernel(const double2 *__restrict__ img, long long n,
+                                                 const double *__restrict__ part, int nparts,
+                                                 double *__restrict__ dB) {
+    const DbScale s = db_scale(image_max2(part, nparts));
+    const bool vec = (reinterpret_cast<uintptr_t>(dB) & 15) == 0;
+    const long long stride = 2LL * gridDim.x * blockDim.x;
+    for (long long i = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x); i < n; i += stride) {
+        if (i + 1 < n) {
+            const double2 z0 = img[i], z1 = img[i + 1];
+            const double d0 = db_of(z0, s), d1 = db_of(z1, s);
+            if (vec) {
+                *reinterpret_cast<double2 *>(dB + i) = make_double2(d0, d1);
+            } else {
+                dB[i] = d0;
+                dB[i + 1] = d1;
+            }
+        } else {
+            dB[i] = db_of(img[i], s);
         }
-        const double a = sqrt(z.x * z.x + z.y * z.y);
-        const double d = 10.0 * (log(a / m) / kLn10F32);
-        dB[i] = d;
-        if (u8) u8[i] = to_u8(d, lo, hi);
     }
 }
 
@@ -135,26 +184,40 @@ __device__ __forceinline__ void u8_quad(const double2 *__restrict__ img, long lo
     }
 }
 
-// blockIdx.y = job; jobs without an u8 output return at once.  Each thread
-// converts four neighbouring pixels at a time.
-__global__ void batch_u8_kernel(const DevJob *__restrict__ jobs) {
-    const DevJob &jb = jobs[blockIdx.y];
-    if (!jb.out_u8) return;
-    const double m = __longlong_as_double((long long)jb.sc->maxabs);
-    const long long n = (long long)jb.nu * jb.nv;
-    const U8Scale us = u8_scale(m, jb.dB_min, jb.dB_max);
-    const bool vec = ((reinterpret_cast<uintptr_t>(jb.out_u8) & 3) == 0);
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; 4 * q < n; q += stride)
-        u8_quad(jb.out, n, 4 * q, jb.out_u8, vec, us);
+// The u8 images of a batch in chunks of kU8Chunk pixels, a job's chunks from
+// jb.u8_chunk0 on; each CTA takes a run of chunks, whichever jobs they fall
+// into (a fixed number of CTAs per job left the largest images of a mix to
+// few: 12 jobs of 256^2 to 1024^2 pixels 92 -> 81 us).  Each thread converts
+// four neighbouring pixels.
+__global__ void __launch_bounds__(256) batch_u8_kernel(const DevJob *__restrict__ jobs, int njobs, long long total,
+                                                       long long per) {
+    const long long c0 = blockIdx.x * per, c1 = c0 + per < total ? c0 + per : total;
+    int cur = -1;
+    U8Scale us;
+    for (long long c = c0; c < c1; ++c) {
+        // the last job that starts at or before chunk c (jobs without an u8
+        // image have no chunks)
+        int before = 0;
+        for (int j0 = 0; j0 < njobs; j0 += 256) {
+            const int j = j0 + (int)threadIdx.x;
+            before += __syncthreads_count(j < njobs && jobs[j].u8_chunk0 <= c);
+        }
+        const DevJob &jb = jobs[before - 1];
+        if (cur != before - 1) {
+            cur = before - 1;
+            us = u8_scale(__longlong_as_double((long long)jb.sc->maxabs), jb.dB_min, jb.dB_max);
+        }
+        const long long n = (long long)jb.nu * jb.nv, i0 = (c - jb.u8_chunk0) * kU8Chunk + 4 * threadIdx.x;
+        if (i0 < n) u8_quad(jb.out, n, i0, jb.out_u8, (reinterpret_cast<uintptr_t>(jb.out_u8) & 3) == 0, us);
+    }
 }
 
-// The same conversion for one image given by its pointer and a max|z| from
-// maxabs_kernel.
-__global__ void img_u8_kernel(const double2 *__restrict__ img, long long n,
-                              const unsigned long long *__restrict__ maxbits, uint8_t *__restrict__ u8,
-                              double lo, double hi) {
-    const U8Scale us = u8_scale(__longlong_as_double((long long)*maxbits), lo, hi);
+// The same conversion for one image given by its pointer and the partial
+// maxima of max2_kernel.
+__global__ void __launch_bounds__(256) img_u8_kernel(const double2 *__restrict__ img, long long n,
+                                                     const double *__restrict__ part, int nparts,
+                                                     uint8_t *__restrict__ u8, double lo, double hi) {
+    const U8Scale us = u8_scale(sqrt(image_max2(part, nparts)), lo, hi);
     const bool vec = ((reinterpret_cast<uintptr_t>(u8) & 3) == 0);
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; 4 * q < n; q += stride)
@@ -179,22 +242,24 @@ long long resident_ctas(K kernel, int *cache) {
     *cache = occ * sms;
     return *cache;
 }
-int g_maxabs_ctas = 0, g_img_u8_ctas = 0, g_batch_u8_ctas = 0;
+int g_max2_ctas = 0, g_img_u8_ctas = 0, g_batch_u8_ctas = 0, g_db_ctas = 0;
 
-}  // namespace
-
-cudaError_t launch_maxabs(const double2 *img, long long n, unsigned long long *d_max, cudaStream_t st) {
+// the partial maxima of an image; their number
+int launch_max2(const double2 *img, long long n, double *part, cudaStream_t st) {
     // at least eight pixels a thread (two steps of four loads), at most one
     // wave of resident CTAs
     const long long b = std::max<long long>(
-        1, std::min<long long>((n + 2047) / 2048, resident_ctas(maxabs_kernel, &g_maxabs_ctas)));
-    maxabs_kernel<<<(unsigned)b, 256, 0, st>>>(img, n, d_max);
-    return cudaGetLastError();
+        1, std::min<long long>({(n + 2047) / 2048, resident_ctas(max2_kernel, &g_max2_ctas), (long long)kMaxParts}));
+    max2_kernel<<<(unsigned)b, 256, 0, st>>>(img, n, part);
+    return (int)b;
 }
 
-cudaError_t launch_db_u8(const double2 *img, long long n, const unsigned long long *d_max, double *dB,
-                         uint8_t *u8, double lo, double hi, cudaStream_t st) {
-    db_u8_kernel<<<grid_for(n), 256, 0, st>>>(img, n, d_max, dB, u8, lo, hi);
+}  // namespace
+
+cudaError_t launch_db(const double2 *img, long long n, double *part, double *dB, cudaStream_t st) {
+    const int np = launch_max2(img, n, part, st);
+    const long long b = std::max<long long>(1, std::min<long long>((n + 511) / 512, resident_ctas(db_kernel, &g_db_ctas)));
+    db_kernel<<<(unsigned)b, 256, 0, st>>>(img, n, part, np, dB);
     return cudaGetLastError();
 }
 
@@ -204,22 +269,22 @@ cudaError_t launch_u8_from_db(const double *dB, long long n, double lo, double h
     return cudaGetLastError();
 }
 
-cudaError_t launch_img_u8(const double2 *img, long long n, const unsigned long long *d_max, uint8_t *u8,
-                          double lo, double hi, cudaStream_t st) {
+cudaError_t launch_img_u8(const double2 *img, long long n, double *part, uint8_t *u8, double lo, double hi,
+                          cudaStream_t st) {
+    const int np = launch_max2(img, n, part, st);
     // one wave of resident CTAs, four pixels per thread and step
     const long long bx = std::max<long long>(
         1, std::min<long long>((n / 4 + 255) / 256, resident_ctas(img_u8_kernel, &g_img_u8_ctas)));
-    img_u8_kernel<<<(unsigned)bx, 256, 0, st>>>(img, n, d_max, u8, lo, hi);
+    img_u8_kernel<<<(unsigned)bx, 256, 0, st>>>(img, n, part, np, u8, lo, hi);
     return cudaGetLastError();
 }
 
-cudaError_t launch_batch_u8(const DevJob *d_jobs, int njobs, long long max_pixels, cudaStream_t st) {
-    // one wave of resident CTAs over the whole batch
-    long long bx = (max_pixels / 4 + 255) / 256;
-    const long long cap =
-        std::max<long long>(1, (resident_ctas(batch_u8_kernel, &g_batch_u8_ctas) + njobs - 1) / njobs);
-    bx = std::max<long long>(1, std::min(bx, cap));
-    batch_u8_kernel<<<dim3((unsigned)bx, njobs), 256, 0, st>>>(d_jobs);
+cudaError_t launch_batch_u8(const DevJob *d_jobs, int njobs, long long chunks, cudaStream_t st) {
+    if (chunks <= 0) return cudaSuccess;
+    // at most one wave of resident CTAs over the whole batch
+    const long long cap = resident_ctas(batch_u8_kernel, &g_batch_u8_ctas);
+    const long long per = (chunks + cap - 1) / cap;
+    batch_u8_kernel<<<(unsigned)((chunks + per - 1) / per), 256, 0, st>>>(d_jobs, njobs, chunks, per);
     return cudaGetLastError();
 }
 

@@ -145,6 +145,7 @@ void describe_job(const sarbp_job &j, int prec, int tile_x, int tile_y, DevJob &
     dj.out_u8 = j.out_u8;
     dj.dB_min = j.dB_min;
     dj.dB_max = j.dB_max;
+    dj.u8_chunk0 = 0;
     dj.host_status = nullptr;
     dj.chunked = 0;
     dj.acc = nullptr;
@@ -539,6 +540,7 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
     char *h = static_cast<char *>(host_meta_.ptr);
     char *d = static_cast<char *>(meta_.ptr);
 
+    long long u8_total = 0;  // chunks of the u8 kernel
     DevJob one;
     DevJob *hj = single ? &one : reinterpret_cast<DevJob *>(h + o_jobs);
     for (int i = 0; i < njobs; ++i) {
@@ -558,6 +560,8 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         dj.pulse = reinterpret_cast<double4 *>(sbase + lay[i].pulse);
         dj.sc = reinterpret_cast<JobScalars *>(sbase) + i;
         dj.host_status = static_cast<int *>(status_pin_.ptr) + (size_t)i * kStatusWords;
+        dj.u8_chunk0 = u8_total;
+        if (j.out_u8) u8_total += u8_chunks((long long)j.nu * j.nv);
         dj.nsplit = nsplit[i];
         dj.parts = nsplit[i] > 1 ? reinterpret_cast<float2 *>(sbase + lay[i].parts) : nullptr;
     }
@@ -744,14 +748,8 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         for (int g = 0; g < slabs->nslabs; ++g)
             if ((e = cudaEventRecord(slabs->done[g], st)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
     if ((e = rec(4)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
-    bool any_u8 = false;
-    long long max_px = 0;
-    for (int i = 0; i < njobs; ++i) {
-        any_u8 = any_u8 || jobs[i].out_u8;
-        max_px = std::max(max_px, (long long)jobs[i].nu * jobs[i].nv);
-    }
-    if (any_u8) {
-        e = launch_batch_u8(d_jobs, njobs, max_px, st);
+    if (u8_total > 0) {
+        e = launch_batch_u8(d_jobs, njobs, u8_total, st);
         if (e != cudaSuccess) return cuda_fail(e, "u8 launch");
         dev_->launches++;
         if ((e = rec(5)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");

@@ -1,0 +1,58 @@
+"""dB and u8 images at the edges of their f32 and f64 ranges; GPU tests."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch():
+    return pytest.importorskip("torch")
+
+
+def _images(rng):
+    z = rng.normal(size=(37, 53)) + 1j * rng.normal(size=(37, 53))
+    bright = z.copy()
+    bright[5, 7] *= 1e4  # most pixels far below the display range
+    mixed = z * 10.0 ** rng.uniform(-20, 0, size=z.shape)
+    mixed[::3] = 0.0
+    return {"speckle": z, "bright": bright, "mixed": mixed, "one": z[:1, :1], "odd": bright[:1, :1023 // 23],
+            "tiny": bright * 1e-30, "huge": mixed * 1e30, "f32_min": mixed * 1e-19, "f64_min": z * 1e-160,
+            "f64_max": z * 1e150, "equal": np.full((8, 9), 3.0 - 4.0j), "zero": np.zeros((4, 6), np.complex128)}
+
+
+@pytest.mark.parametrize("lo,hi", [(-45.0, 0.0), (-30.0, -10.0), (-400.0, 5.0)])
+@pytest.mark.parametrize("name", sorted(_images(np.random.default_rng(0))))
+def test_db_and_u8_match_oracle(ctx, oracle, torch, name, lo, hi):
+    """u8 exactly the oracle's, from the image at once and through the dB
+    image; dB within 1e-12 of it (three roundings of the square, times 5 / ln
+    10, are 8e-16; a square below 1e-290 is left to the oracle's formula)."""
+    img = np.ascontiguousarray(_images(np.random.default_rng(3))[name], np.complex128)
+    nv, nu = img.shape
+    want_dB = oracle.img_output_to_dB(img)
+    want = oracle.img_output_u8(want_dB, lo, hi)
+    dB = ctx.img_output_to_dB(img)
+    fine = np.isfinite(want_dB)
+    assert np.array_equal(fine, np.isfinite(dB)) and np.array_equal(np.isnan(want_dB), np.isnan(dB))
+    if fine.any():
+        assert np.abs(dB[fine] - want_dB[fine]).max() < 1e-12 and dB[fine].max() == want_dB[fine].max() == 0.0
+    assert np.array_equal(ctx.img_output_u8(dB, lo, hi), want)
+    t = torch.from_numpy(img.view(np.float64)).cuda()
+    for off in (0, 1):  # aligned and unaligned destination
+        out = torch.zeros(nu * nv + 8, dtype=torch.uint8, device="cuda")
+        ctx.img_output_u8_from_img_device(t.data_ptr(), nu, nv, lo, hi, out.data_ptr() + off)
+        ctx.synchronize()
+        assert np.array_equal(out.cpu().numpy()[off:off + nu * nv].reshape(nv, nu), want)
+
+
+def test_unaligned_db_destination(ctx, sb, torch):
+    from sarbp_b200._lib import check, lib
+    img = torch.randn(5, 7, 2, dtype=torch.float64, device="cuda")
+    a, b = torch.zeros(40, dtype=torch.float64, device="cuda"), torch.zeros(40, dtype=torch.float64, device="cuda")
+    p = lambda t, o=0: ctypes.c_void_p(t.data_ptr() + o)
+    check(lib().sarbp_img_output_to_dB_device(ctx.handle, p(img), 7, 5, p(a)))
+    check(lib().sarbp_img_output_to_dB_device(ctx.handle, p(img), 7, 5, p(b, 8)))
+    ctx.synchronize()
+    assert torch.equal(a[:35], b[1:36]) and float(a[35]) == 0.0 == float(b[36])
