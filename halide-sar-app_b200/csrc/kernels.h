@@ -99,12 +99,13 @@ struct ResizePlan {
     int rows, cols, orows, ocols;
     double zoom[2];        // input / output extent per axis
     int radius[2];         // Gaussian radius per axis; -1: axis not filtered
-    int woff[2];           // offset of each axis's weights w[0..radius] in d_weights
-    const double *d_weights;
+    int woff[2];           // offset of each axis's weights w[0..radius] in weights
+    const double *weights; // host
+    double *d_weights;     // room for them on the device
     void *d_taps;          // (orows + ocols) * 32 bytes of scratch: the zoom's taps per index
 };
 cudaError_t launch_resize(const ResizePlan &p, const void *in, void *out, void *tmp_a, void *tmp_b,
-                          double *bounds, cudaStream_t st);
+                          double *bounds, cudaStream_t st, int *launches);
 
 // peaks.cu
 cudaError_t measure_peaks(int num_sms, cudaStream_t st, double *ffma_per_s, double *mufu_per_s);

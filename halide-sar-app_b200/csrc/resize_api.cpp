@@ -93,15 +93,13 @@ int resize_enqueue(sarbp_ctx *ctx, int elem_bytes, int ncomp, const void *in, in
     if (e != cudaSuccess) return cuda_fail(e, "resize: scratch");
     char *base = static_cast<char *>(ctx->resize_buf.ptr);
     double *d_w = reinterpret_cast<double *>(base), *d_b = reinterpret_cast<double *>(base + b_w);
-    if (!weights.empty())
-        e = cudaMemcpyAsync(d_w, weights.data(), weights.size() * sizeof(double), cudaMemcpyHostToDevice,
-                            ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "resize: weights");
+    p.weights = weights.data();
     p.d_weights = d_w;
     p.d_taps = base + b_w + b_b + 2 * a256(n_in);
-    e = launch_resize(p, in, out, base + b_w + b_b, base + b_w + b_b + a256(n_in), d_b, ctx->stream);
+    int launches = 0;
+    e = launch_resize(p, in, out, base + b_w + b_b, base + b_w + b_b + a256(n_in), d_b, ctx->stream, &launches);
     if (e != cudaSuccess) return cuda_fail(e, "resize launch");
-    ctx->dev.launches += 4 + (p.radius[0] >= 0) + (p.radius[1] >= 0);
+    ctx->dev.launches += launches;
     return SARBP_OK;
 }
 

@@ -75,3 +75,63 @@ def test_resize_tool_on_afrl_files(ctx, afrl_input, tmp_path):
         _check(got["k_r"], k_r)
         _check(got["phs"], phs)
         _check(got["pos"], pos)
+
+
+def _device(ctx, torch, a, shape, shift=0, over=False):
+    """sarbp_resize_device of a [rows][cols][ncomp] array; `shift` puts the
+    output that many elements off its alignment, `over` over the input."""
+    import ctypes
+
+    from sarbp_b200._lib import check, lib
+    t = torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    n = shape[0] * shape[1] * a.shape[2]
+    buf = torch.zeros(max(n, t.numel()) + 4, dtype=t.dtype, device="cuda")
+    src = t
+    if over:
+        buf[:t.numel()] = t.reshape(-1)
+        src = buf
+    p = lambda x, o=0: ctypes.c_void_p(x.data_ptr() + o * x.element_size())
+    check(lib().sarbp_resize_device(ctx.handle, t.element_size(), a.shape[2], p(src), a.shape[0], a.shape[1],
+                                    shape[0], shape[1], p(buf, shift)))
+    ctx.synchronize()
+    return buf[shift:shift + n].reshape(shape[0], shape[1], a.shape[2]).cpu().numpy()
+
+
+# one output row or column, tiles and remainders, the largest filters of the
+# tile kernel and the ones beyond it, one axis each way, single rows and columns
+@pytest.mark.parametrize("shape_in,shape_out", [
+    ((300, 260), (150, 130)), ((131, 129), (33, 127)), ((500, 40), (140, 40)), ((520, 64), (130, 16)),
+    ((40, 900), (41, 110)), ((64, 700), (64, 80)), ((33, 70), (200, 515)), ((1, 1000), (1, 260)), ((1000, 1), (301, 1)),
+    ((2, 2), (5, 5)), ((7, 5), (1, 1)), ((90, 90), (89, 91)), ((257, 300), (70, 1)),
+])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("nc", [1, 2])
+def test_tile_kernel_matches_oracle_and_steps(ctx, shape_in, shape_out, dtype, nc):
+    import torch
+    from resize_oracle import sk_resize
+    a = np.random.default_rng(11).normal(size=shape_in + (nc,)).astype(dtype)
+    got = _device(ctx, torch, a, shape_out)
+    for k in range(nc):
+        _check(got[..., k], sk_resize(a[..., k], shape_out))
+    # an output over its input is formed step by step
+    steps = _device(ctx, torch, a, shape_out, over=True) if np.prod(shape_out) <= np.prod(shape_in) else got
+    tol = (1e-6 if dtype == np.float32 else 1e-14) * np.abs(a).max()
+    np.testing.assert_allclose(got, steps, rtol=0, atol=tol)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("shape_out", [(30, 21), (100, 90), (61, 20)])
+def test_tile_kernel_clips_like_the_steps(ctx, dtype, shape_out):
+    """Constant arrays stay constant; NaN and infinities come out as the
+    step-by-step kernels leave them (clipped to the extremes)."""
+    import torch
+    c = np.full((61, 43, 2), 0.1, dtype)
+    assert np.array_equal(_device(ctx, torch, c, shape_out), np.full(shape_out + (2,), 0.1, dtype))
+    a = np.random.default_rng(2).normal(size=(61, 43, 2)).astype(dtype)
+    a[5, 7, 0] = np.nan
+    a[40, 30, 1] = np.inf
+    a[0, 0, 1] = -np.inf
+    for b in (a, np.full_like(a, np.nan)):
+        got, want = _device(ctx, torch, b, shape_out), _device(ctx, torch, b, shape_out, shift=1)
+        tol = (1e-6 if dtype == np.float32 else 1e-14) * 5
+        np.testing.assert_allclose(got, want, rtol=0, atol=tol)
