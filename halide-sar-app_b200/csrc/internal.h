@@ -118,9 +118,11 @@ struct DevJob {
     // pulse parts: a job whose tiles leave resident CTAs idle has each tile
     // formed as nsplit items over consecutive pulse ranges (part_range);
     // each item stores its sums into slice `part` of parts ([nsplit][nv][nu],
-    // pixel-row order), and the last of a tile's items adds the slices in order
-    // and applies the final phase.  nsplit <= 1: one item per tile.
+    // pixel-row order), and the last of a tile's items (sum_parts), or else the
+    // combine kernel, adds the slices in order and applies the final phase.
+    // nsplit <= 1: one item per tile.
     int nsplit;
+    int sum_parts;
     float2 *parts;
 };
 

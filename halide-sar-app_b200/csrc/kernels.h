@@ -91,6 +91,10 @@ cudaError_t launch_tile_records(const DevJob *d_jobs, const WorkItem *d_items, i
 cudaError_t launch_chunk_setup(const DevJob &job, DevJob *d_dst, const double4 *pulse, const float *wP, int P, int q0,
                                int *counters, cudaStream_t st);
 cudaError_t launch_finalize(const DevJob &job, long long npix, int num_sms, cudaStream_t st);
+// jobs d_list[0 .. nlist) of d_jobs, formed in pulse parts without sum_parts:
+// sum of the parts times the final phase into out (row flip), max |z|
+cudaError_t launch_combine_parts(const DevJob *d_jobs, const int *d_list, int nlist, long long max_pixels,
+                                 int num_sms, cudaStream_t st);
 
 // resize.cu (the reference's data/resize.py resampling)
 struct ResizePlan {

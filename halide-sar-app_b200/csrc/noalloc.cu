@@ -237,6 +237,7 @@ extern "C" int sarbp_backprojection_noalloc(const sarbp_job *job, void *cuda_str
     dj.dB_min = j.dB_min;
     dj.dB_max = j.dB_max;
     dj.nsplit = nsplit;
+    dj.sum_parts = 1;
     dj.parts = nsplit > 1 ? reinterpret_cast<float2 *>(sb + o_parts) : nullptr;
 
     DevJob *d_job = reinterpret_cast<DevJob *>(sb + o_job);

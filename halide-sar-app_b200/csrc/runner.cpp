@@ -150,6 +150,7 @@ void describe_job(const sarbp_job &j, int prec, int tile_x, int tile_y, DevJob &
     dj.chunked = 0;
     dj.acc = nullptr;
     dj.nsplit = 1;
+    dj.sum_parts = 0;
     dj.parts = nullptr;
 }
 
@@ -515,16 +516,28 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         nrows_total += kv.second.size();
     }
 
+    // a tile's parts are added by its last item where every CTA has one item
+    const int resident_bp = any_split ? bp_max_active_blocks(L) * dev_->num_sms : 0;
+    const bool sum_parts = any_split && L.persistent && nitems <= (size_t)resident_bp;
+    std::vector<int> combine;  // jobs that need the combine kernel
+    long long combine_px = 0;
+    for (int i = 0; i < njobs; ++i)
+        if (nsplit[i] > 1 && !sum_parts) {
+            combine.push_back(i);
+            combine_px = std::max(combine_px, (long long)jobs[i].nu * jobs[i].nv);
+        }
+
     // ---- meta block: [DevJob][RowItem...][WorkItem...][tile WorkItem...]
-    // [counters] (the tile list only when a job of several is split: the work
+    // [combine list][counters] (the tile list only when a job of several is split: the work
     // items are then not one per tile) ----
     const size_t o_jobs = 0;
     const size_t o_rows = align_up(o_jobs + (size_t)njobs * sizeof(DevJob), 256);
     const size_t o_items = align_up(o_rows + nrows_total * sizeof(RowItem), 256);
     const size_t o_tiles = align_up(o_items + nitems * sizeof(WorkItem), 256);
-    const size_t o_cnt = align_up(o_tiles + tiles.size() * sizeof(WorkItem), 256);
+    const size_t o_comb = align_up(o_tiles + tiles.size() * sizeof(WorkItem), 256);
+    const size_t o_cnt = align_up(o_comb + combine.size() * sizeof(int), 256);
     const size_t cnt_bytes = slabs ? kBpCounterBytes * (size_t)slabs->nslabs : (size_t)kBpDealBytes;
-    const size_t meta_bytes = o_cnt + cnt_bytes;
+    const size_t meta_bytes = o_cnt + cnt_bytes + sizeof(int);
     if (for_graph && ((!single && host_meta_.cap < meta_bytes) || meta_.cap < meta_bytes))
         return fail(SARBP_ERR_STATE, "graph capture needs a prior run of the same jobs");
     if (!single) {
@@ -563,6 +576,7 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         dj.u8_chunk0 = u8_total;
         if (j.out_u8) u8_total += u8_chunks((long long)j.nu * j.nv);
         dj.nsplit = nsplit[i];
+        dj.sum_parts = sum_parts;
         dj.parts = nsplit[i] > 1 ? reinterpret_cast<float2 *>(sbase + lay[i].parts) : nullptr;
     }
     // The caller's inputs may still be on their way on the slabs' copy stream
@@ -574,6 +588,7 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
             std::memcpy(hr + g.first, rows[g.logN].data(), g.count * sizeof(RowItem));
         std::memcpy(h + o_items, items.data(), items.size() * sizeof(WorkItem));
         std::memcpy(h + o_tiles, tiles.data(), tiles.size() * sizeof(WorkItem));
+        std::memcpy(h + o_comb, combine.data(), combine.size() * sizeof(int));
         e = cudaMemcpyAsync(d, h, meta_bytes, cudaMemcpyHostToDevice, ms);
         if (e != cudaSuccess) return cuda_fail(e, "copying descriptors");
     }
@@ -587,6 +602,8 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
     // (one job's items begin with part 0 of every tile)
     const WorkItem *d_tiles = single || !any_split ? d_items : reinterpret_cast<const WorkItem *>(d + o_tiles);
     int *d_cnt = reinterpret_cast<int *>(d + o_cnt);
+    // (one job's counters are followed by a zero: its index in the list)
+    const int *d_comb = single ? d_cnt + cnt_bytes / sizeof(int) : reinterpret_cast<const int *>(d + o_comb);
 
     // twiddle tables first (a one-time synchronous upload per N_fft; a
     // four-step N_fft also needs the tables of its two sub-lengths)
@@ -606,7 +623,7 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
     if ((e = rec(0)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
     if (single) {
         e = launch_prep_single(one, SingleLists{d_jobs, d_items, (int)ntile_items, (int)nitems, d_rows,
-                                                (int)nrows_total, d_cnt, (int)(cnt_bytes / sizeof(int))}, st);
+                                                (int)nrows_total, d_cnt, (int)(cnt_bytes / sizeof(int)) + 1}, st);
         if (e != cudaSuccess) return cuda_fail(e, "set-up launch");
     } else {
         launch_prep(d_jobs, njobs, st);
@@ -737,6 +754,11 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         }
         e = launch_backproject(L, d_jobs, d_items, (int)nitems, d_cnt, st);
         if (e != cudaSuccess) return cuda_fail(e, "backprojection launch");
+        dev_->launches++;
+    }
+    if (!combine.empty()) {
+        e = launch_combine_parts(d_jobs, d_comb, (int)combine.size(), combine_px, dev_->num_sms, st);
+        if (e != cudaSuccess) return cuda_fail(e, "pulse-part combine launch");
         dev_->launches++;
     }
     for (int i : naive) {
