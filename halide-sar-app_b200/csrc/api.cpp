@@ -108,6 +108,14 @@ int run_host_job(sarbp_ctx *ctx, const float *phs, int S, int P, const float *k_
     int tile_x = 0, tile_y = 0, nslabs = 0, row0[sarbp_ctx::kMaxSlabs + 1] = {};
     slab_plan(opts, precision, nu, nv, &tile_x, &tile_y, &nslabs, row0);
     cudaStream_t cin = nslabs ? ctx->copy_in : st;
+    // pageable arrays go through page-locked slots (see hostcopy.h)
+    const size_t n_out = npix * 2 * sizeof(double);
+    const bool stage_r = r && HostStager::wants(r, npix * 3 * sizeof(double));
+    const bool stage_out = HostStager::wants(out, n_out);
+    const HostStager::Session session(&ctx->stager);
+    auto to_device = [&](void *dst, const void *src, size_t n, bool staged) {
+        return staged ? ctx->stager.upload(dst, src, n, cin) : cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, cin);
+    };
     struct Copy { void *dst; const void *src; size_t n; };
     const Copy copies[] = {
         {d_phs, phs, (size_t)S * P * 2 * sizeof(float)},
@@ -121,7 +129,7 @@ int run_host_job(sarbp_ctx *ctx, const float *phs, int S, int P, const float *k_
     };
     for (const Copy &c : copies) {
         if (!c.src) continue;
-        e = cudaMemcpyAsync(c.dst, c.src, c.n, cudaMemcpyHostToDevice, cin);
+        e = to_device(c.dst, c.src, c.n, HostStager::wants(c.src, c.n));
         if (e != cudaSuccess) return cuda_fail(e, "copying inputs to the device");
     }
     SlabSpec spec;
@@ -135,8 +143,7 @@ int run_host_job(sarbp_ctx *ctx, const float *phs, int S, int P, const float *k_
                 const size_t y1 = std::min((size_t)nv, (size_t)row0[g + 1] * tile_y);
                 for (int c = 0; c < 3 && y1 > y0; ++c) {
                     const size_t off = (size_t)c * npix + y0 * (size_t)nu;
-                    cudaError_t ce = cudaMemcpyAsync(d_r + off, r + off, (y1 - y0) * (size_t)nu * sizeof(double),
-                                                     cudaMemcpyHostToDevice, cin);
+                    cudaError_t ce = to_device(d_r + off, r + off, (y1 - y0) * (size_t)nu * sizeof(double), stage_r);
                     if (ce != cudaSuccess) return ce;
                 }
                 cudaError_t ce = cudaEventRecord(ctx->ev_ready[g], cin);
@@ -182,7 +189,9 @@ int run_host_job(sarbp_ctx *ctx, const float *phs, int S, int P, const float *k_
         return rc;
     }
     if (!nslabs) {
-        e = cudaMemcpyAsync(out, d_out, npix * 2 * sizeof(double), cudaMemcpyDeviceToHost, st);
+        e = stage_out ? ctx->stager.download(out, d_out, n_out, st)
+                      : cudaMemcpyAsync(out, d_out, n_out, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess && stage_out) e = ctx->stager.drain();
         if (e != cudaSuccess) return cuda_fail(e, "copying the image to the host");
         return ctx->runner->check_status(st);
     }
@@ -194,10 +203,12 @@ int run_host_job(sarbp_ctx *ctx, const float *phs, int S, int P, const float *k_
         if ((e = cudaStreamWaitEvent(ctx->copy_out, ctx->ev_done[g], 0)) != cudaSuccess)
             return cuda_fail(e, "cudaStreamWaitEvent");
         const size_t off = ((size_t)nv - y1) * (size_t)nu * 2;
-        e = cudaMemcpyAsync(out + off, d_out + off, (y1 - y0) * (size_t)nu * 2 * sizeof(double),
-                            cudaMemcpyDeviceToHost, ctx->copy_out);
+        const size_t n = (y1 - y0) * (size_t)nu * 2 * sizeof(double);
+        e = stage_out ? ctx->stager.download(out + off, d_out + off, n, ctx->copy_out)
+                      : cudaMemcpyAsync(out + off, d_out + off, n, cudaMemcpyDeviceToHost, ctx->copy_out);
         if (e != cudaSuccess) return cuda_fail(e, "copying the image to the host");
     }
+    if (stage_out && (e = ctx->stager.drain()) != cudaSuccess) return cuda_fail(e, "copying the image to the host");
     if ((e = cudaEventRecord(ctx->ev_out, ctx->copy_out)) != cudaSuccess ||
         (e = cudaStreamWaitEvent(st, ctx->ev_out, 0)) != cudaSuccess)
         return cuda_fail(e, "ordering output copies");
@@ -265,6 +276,7 @@ int sarbp_ctx_destroy(sarbp_ctx *ctx) {
     cudaSetDevice(ctx->dev.device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     ctx->runner.reset();
+    ctx->stager.release();
     ctx->io.release();
     ctx->out_aux.release();
     ctx->resize_buf.release();

@@ -7,6 +7,7 @@
 #include <memory>
 #include <string>
 
+#include "hostcopy.h"
 #include "runner.h"
 #include "sarbp_b200.h"
 
@@ -23,6 +24,7 @@ struct sarbp_ctx {
     // and the events that pipeline row slabs between them
     static constexpr int kMaxSlabs = 12;
     cudaStream_t copy_in = nullptr, aux = nullptr, copy_out = nullptr;
+    sarbp::HostStager stager;  // copies of pageable buffers
     cudaEvent_t ev_out = nullptr;
     cudaEvent_t ev_ready[kMaxSlabs] = {}, ev_done[kMaxSlabs] = {};
 };
