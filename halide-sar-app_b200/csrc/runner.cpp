@@ -351,14 +351,16 @@ size_t Runner::job_scratch_bytes(const sarbp_job &j, const sarbp_opts *opts, boo
 }
 
 Runner::~Runner() {
-    if (side_) cudaStreamSynchronize(side_);
+    for (cudaStream_t s : {side_, side_high_})
+        if (s) cudaStreamSynchronize(s);
     scratch_.release();
     meta_.release();
     host_meta_.release();
     status_pin_.release();
     if (meta_done_) cudaEventDestroy(meta_done_);
     if (front_done_) cudaEventDestroy(front_done_);
-    if (side_) cudaStreamDestroy(side_);
+    for (cudaStream_t s : {side_, side_high_})
+        if (s) cudaStreamDestroy(s);
     if (fork_) cudaEventDestroy(fork_);
     if (join_) cudaEventDestroy(join_);
 }
@@ -631,25 +633,39 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
     dev_->launches++;
     if ((e = rec(1)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
     const bool slabbed = slabs && nitems > 0 && prec[0] != SARBP_PREC_NAIVE;
-    // Range compression beside the tile geometry: both read only the
-    // set-up's tables, and the backprojection waits for both.  Each kernel
-    // fills the SMs on its own, so they mostly fill each other's tails
-    // (5.988 -> 5.979 ms per 2048^2 x 1999 step).  Not while the context
-    // times its stages (each stage then runs alone), and not for row slabs
-    // (their geometry already runs beside the backprojection).
+    // The tile geometry beside the range compression: both read only the
+    // set-up's tables, and the backprojection waits for both.  One of them runs
+    // on a second stream and is launched first: the geometry while its CTAs fit
+    // on the SMs at once (4 per SM) and either occupy all of them or would wait
+    // behind range compression's (4 jobs of 128^2 and 256^2 pixels, 112 tiles,
+    // 1282 CTAs of rows: 147 us replayed behind it, 135 ahead; 512^2: 148 and
+    // 143); range compression otherwise, in several launches above all (6 jobs,
+    // 768 tiles: 406 us first, 417 second; 4 jobs with two row lengths 383 and
+    // 393).  The second stream has high priority in between the images whose
+    // kernels leave SMs free anyway (256^2: 56 us without, 57.5 with) and those
+    // that fill them many times over (2048^2: 5.73 ms and 5.74; 1000x731: 540 us
+    // and 538; 922x1062 x 144: 161 and 158).  Not while the context times its
+    // stages (each stage then runs alone), and not for row slabs (their geometry
+    // already runs beside the backprojection).
     const bool side = !rc_only && !slabbed && nitems > 0 && !row_groups.empty() &&
                       !(stage_events && dev_->timing && !for_graph);
-    cudaStream_t rs = st;
+    const size_t sms = (size_t)dev_->num_sms;
+    const bool geometry_first = side && row_groups.size() == 1 && ntile_items <= 4 * sms &&
+                                (ntile_items >= sms || (row_groups[0].count << row_groups[0].logN) > 5 * sms * 4096);
+    const bool crowded = side && (geometry_first || (ntile_items >= sms && ntile_items <= 16 * sms));
+    cudaStream_t &second = crowded ? side_high_ : side_;
     if (side) {
-        if (!side_ && (e = cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking)) != cudaSuccess)
+        int least = 0, greatest = 0;
+        if (!second && ((e = cudaDeviceGetStreamPriorityRange(&least, &greatest)) != cudaSuccess ||
+                        (e = cudaStreamCreateWithPriority(&second, cudaStreamNonBlocking, crowded ? greatest : least)) !=
+                            cudaSuccess))
             return cuda_fail(e, "creating a stream");
         if (!fork_ && (e = cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming)) != cudaSuccess)
             return cuda_fail(e, "cudaEventCreate");
         if (!join_ && (e = cudaEventCreateWithFlags(&join_, cudaEventDisableTiming)) != cudaSuccess)
             return cuda_fail(e, "cudaEventCreate");
-        if ((e = cudaEventRecord(fork_, st)) != cudaSuccess || (e = cudaStreamWaitEvent(side_, fork_, 0)) != cudaSuccess)
-            return cuda_fail(e, "ordering range compression");
-        rs = side_;
+        if ((e = cudaEventRecord(fork_, st)) != cudaSuccess || (e = cudaStreamWaitEvent(second, fork_, 0)) != cudaSuccess)
+            return cuda_fail(e, "ordering range compression and tile geometry");
     }
     // the main stream waits for the side stream before the backprojection,
     // and on every return in between (nothing may outlive the batch there)
@@ -663,7 +679,13 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
             return r;
         }
         ~Join() { now(); }
-    } join{st, side_, side ? join_ : nullptr};
+    } join{st, second, side ? join_ : nullptr};
+    auto tile_geometry = [&](cudaStream_t s) {
+        dev_->launches++;
+        return launch_tile_setup(d_jobs, d_tiles, (int)ntile_items, L.tile_x * L.tile_y, s);
+    };
+    if (geometry_first && (e = tile_geometry(second)) != cudaSuccess) return cuda_fail(e, "tile geometry launch");
+    const cudaStream_t rs = side && !geometry_first ? second : st;
     for (size_t g = 0; g < row_groups.size(); ++g) {
         const int logN = row_groups[g].logN;
         const size_t first = row_groups[g].first, count = row_groups[g].count;
@@ -722,12 +744,8 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
                 return cuda_fail(e, "cudaStreamWaitEvent");
         nitems = 0;  // formed above
     }
-    if (nitems > 0) {
-        e = launch_tile_setup(d_jobs, d_tiles, (int)ntile_items, L.tile_x * L.tile_y, st);
-        if (e != cudaSuccess) return cuda_fail(e, "tile geometry launch");
-        dev_->launches += 1;
-    }
-    if ((e = join.now()) != cudaSuccess) return cuda_fail(e, "ordering range compression");
+    if (nitems > 0 && !geometry_first && (e = tile_geometry(st)) != cudaSuccess) return cuda_fail(e, "tile geometry launch");
+    if ((e = join.now()) != cudaSuccess) return cuda_fail(e, "ordering range compression and tile geometry");
     if (!slabbed && (e = rec(3)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
     if (nitems > 0) {
         if (L.persistent) {
