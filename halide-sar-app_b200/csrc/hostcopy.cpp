@@ -1,6 +1,8 @@
 // hostcopy.cpp -- see hostcopy.h.
 #include "hostcopy.h"
 
+#include <unistd.h>
+
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
@@ -8,7 +10,13 @@
 namespace sarbp {
 
 namespace {
-inline void relax() {
+// One turn of a wait: a pause at first, then the core goes to whoever else
+// wants it (other contexts' threads, or a copying thread that lost its core).
+inline void relax(int turn) {
+    if (turn >= 4096) {
+        std::this_thread::yield();
+        return;
+    }
 #if defined(__x86_64__)
     __builtin_ia32_pause();
 #endif
@@ -16,6 +24,10 @@ inline void relax() {
 }  // namespace
 
 CopyThreads::~CopyThreads() {
+    if (started_ && pid_ != getpid()) {  // a forked child has no such threads to join
+        new std::vector<std::thread>(std::move(threads_));
+        return;
+    }
     {
         std::lock_guard<std::mutex> lk(mu_);
         stop_ = true;
@@ -28,6 +40,7 @@ CopyThreads::~CopyThreads() {
 void CopyThreads::begin() {
     if (!started_) {
         started_ = true;
+        pid_ = getpid();
         // half of the cores at most, the caller among them (16 cores: 1.33 ms with 3
         // helpers, 1.23 with 5, 1.18 with 7)
         const int n = std::min(7, (int)std::thread::hardware_concurrency() / 2 - 1);
@@ -58,7 +71,7 @@ bool CopyThreads::take(unsigned gen) {
         unsigned long long v = next_.load(std::memory_order_acquire);
         if ((unsigned)(v >> 32) != gen) return any;
         const unsigned i = (unsigned)v;
-        if (i >= npieces_.load(std::memory_order_relaxed)) return any;
+        if (i >= npieces_.load(std::memory_order_acquire)) return any;
         // (a changed generation fails the exchange, so dst_, src_ and n_ are
         // those of this copy until its last piece is done)
         if (!next_.compare_exchange_weak(v, v + 1, std::memory_order_acq_rel)) continue;
@@ -76,9 +89,11 @@ void CopyThreads::work() {
             cv_.wait(lk, [&] { return stop_ || session_.load(); });
             if (stop_) return;
         }
+        int idle = 0;
         while (session_.load(std::memory_order_relaxed)) {
-            if (!take((unsigned)(next_.load(std::memory_order_acquire) >> 32)))
-                for (int k = 0; k < 32; ++k) relax();
+            if (take((unsigned)(next_.load(std::memory_order_acquire) >> 32))) idle = 0;
+            for (int k = 0; k < 32 && idle < 4096; ++k) relax(idle++);
+            if (idle >= 4096) relax(idle);
         }
     }
 }
@@ -100,7 +115,7 @@ void CopyThreads::copy(char *dst, const char *src, size_t n) {
     npieces_.store((unsigned)pieces, std::memory_order_release);
     next_.store((unsigned long long)gen_ << 32, std::memory_order_release);
     take(gen_);
-    while (left_.load(std::memory_order_acquire) != 0) relax();
+    for (int k = 0; left_.load(std::memory_order_acquire) != 0; k += k < 4096) relax(k);
 }
 
 bool HostStager::wants(const void *p, size_t n) {

@@ -9,6 +9,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <sys/types.h>
 
 #include <atomic>
 #include <condition_variable>
@@ -45,6 +46,7 @@ private:
     const char *src_ = nullptr;
     size_t n_ = 0;
     unsigned gen_ = 0;
+    pid_t pid_ = 0;
 };
 
 class HostStager {
