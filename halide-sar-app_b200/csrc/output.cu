@@ -32,8 +32,9 @@ __device__ __forceinline__ uint8_t to_u8(double v, double lo, double hi) {
 // u8 of one pixel.  The value is decided in f32 (|z|^2 rounded to f32, the
 // accurate logf), whose error is far below 1e-4 of a grey level for display
 // ranges of 0.1 dB and wider; a pixel whose f32 level lands within that
-// margin of an integer or of the clamps, or whose f32 values are not normal
-// numbers, is recomputed with the reference's f64 formula.  Pixels clearly
+// margin of an integer or of the clamps, or whose |z|^2 or ratio to the
+// maximum's is not a normal f32 number (below -190 dB), is recomputed with the
+// reference's f64 formula.  Pixels clearly
 // below dB_min or above dB_max are decided in f32 as well: in a scene of a few
 // bright points that is most of them (12 jobs of 256^2 to 1024^2 pixels, -40
 // dB: 81 us with those in f64, 31 us without).
@@ -58,10 +59,10 @@ __device__ __forceinline__ U8Scale u8_scale(double m, double lo, double hi) {
 
 __device__ __forceinline__ uint8_t u8_of(double2 z, const U8Scale &u) {
     const double a2 = z.x * z.x + z.y * z.y;
-    const float a = (float)a2;
-    const float q = fmaf(u.k, logf(a * u.inv_m2), u.q0);
+    const float a = (float)a2, x = a * u.inv_m2;
+    const float q = fmaf(u.k, logf(x), u.q0);
     const float f = q - floorf(q);
-    if (a >= FLT_MIN && a <= FLT_MAX) {  // (an f32 overflow or underflow says nothing)
+    if (a >= FLT_MIN && a <= FLT_MAX && x >= FLT_MIN) {  // (an f32 overflow or underflow says nothing)
         if (q > u.eps && q < 255.0f - u.eps && f > u.eps && f < 1.0f - u.eps) return (uint8_t)q;
         if (q < -u.eps) return 0;
         if (q > 255.0f + u.eps) return 255;

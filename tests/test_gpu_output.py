@@ -56,3 +56,27 @@ def test_unaligned_db_destination(ctx, sb, torch):
     check(lib().sarbp_img_output_to_dB_device(ctx.handle, p(img), 7, 5, p(b, 8)))
     ctx.synchronize()
     assert torch.equal(a[:35], b[1:36]) and float(a[35]) == 0.0 == float(b[36])
+
+
+# |z|^2 ordinary f32 numbers whose ratio to the maximum's is subnormal or zero there
+@pytest.mark.parametrize("lo,hi", [(-300.0, 0.0), (-500.0, 0.0), (-230.0, -190.0)])
+def test_u8_over_thirty_decades(ctx, oracle, torch, lo, hi):
+    rng = np.random.default_rng(8)
+    img = (rng.normal(size=(61, 47)) + 1j * rng.normal(size=(61, 47))) * 10.0 ** rng.uniform(-20, 9, size=(61, 47))
+    img[0, 0], img[3, 4] = 1e-15, 1e10
+    want = oracle.img_output_u8(oracle.img_output_to_dB(img), lo, hi)
+    t = torch.from_numpy(img.view(np.float64)).cuda()
+    out = torch.zeros(img.size, dtype=torch.uint8, device="cuda")
+    ctx.img_output_u8_from_img_device(t.data_ptr(), 47, 61, lo, hi, out.data_ptr())
+    ctx.synchronize()
+    assert np.array_equal(out.cpu().numpy().reshape(61, 47), want)
+
+
+def test_db_where_the_squares_ratio_leaves_the_f64_range(ctx, oracle):
+    """Pixels down to 280 decades below the maximum: the logarithm of each
+    side is good to an ulp and three roundings follow it (4 x 2.2e-16)."""
+    rng = np.random.default_rng(9)
+    img = (1 + rng.uniform(size=(40, 30)) + 1j * rng.normal(size=(40, 30))) * 10.0 ** rng.uniform(-140, 140, (40, 30))
+    want, got = oracle.img_output_to_dB(img), ctx.img_output_to_dB(img)
+    assert np.isfinite(want).all()
+    np.testing.assert_allclose(got, want, rtol=9e-16, atol=1e-12)
