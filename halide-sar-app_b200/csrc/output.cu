@@ -120,7 +120,8 @@ __device__ __forceinline__ double image_max2(const double *__restrict__ part, in
 // |z|^2 * (1 / m^2), whose three roundings weigh as much with the factor 5 as
 // the reference's with 10 (same error against 64-bit values, 1.1e-16).  The
 // maximum itself stays at exactly 0 and nothing above it; a maximum whose
-// square is not an ordinary number takes the reference's formula.
+// square is not an ordinary number, and a pixel whose ratio to it is none
+// (below -1538 dB), takes the reference's formula.
 // 2048^2: 22 us, 31 before.
 struct DbScale {
     double m2, inv, m;
@@ -131,8 +132,8 @@ __device__ __forceinline__ DbScale db_scale(double m2) {
 }
 __device__ __forceinline__ double db_of(double2 z, const DbScale &s) {
     const double a2 = z.x * z.x + z.y * z.y;
-    if (!s.plain) return 10.0 * (log(sqrt(a2) / s.m) / kLn10F32);
     const double q = a2 == s.m2 ? 1.0 : a2 * s.inv;
+    if (!s.plain || (q < DBL_MIN && a2 > 0.0)) return 10.0 * (log(sqrt(a2) / s.m) / kLn10F32);
     return fmin(5.0 / kLn10F32 * log(q), q == q ? 0.0 : q);
 }
 
