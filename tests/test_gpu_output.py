@@ -80,3 +80,14 @@ def test_db_where_the_squares_ratio_leaves_the_f64_range(ctx, oracle):
     want, got = oracle.img_output_to_dB(img), ctx.img_output_to_dB(img)
     assert np.isfinite(want).all()
     np.testing.assert_allclose(got, want, rtol=9e-16, atol=1e-12)
+
+
+def test_db_error_is_not_above_the_f64_formulas(ctx, oracle):
+    """Against 80-bit values, for the image's own maximum |z|."""
+    rng = np.random.default_rng(10)
+    img = rng.normal(size=(700, 600)) + 1j * rng.normal(size=(700, 600))
+    re, im = img.real.astype(np.longdouble), img.imag.astype(np.longdouble)
+    a = np.sqrt(re * re + im * im)
+    exact = 10 * np.log(a / a.max()) / np.longdouble(np.log(np.float32(10.0)))
+    err = lambda d: float(np.sqrt(np.mean((d - exact) ** 2)))
+    assert err(ctx.img_output_to_dB(img)) <= err(oracle.img_output_to_dB(img))
