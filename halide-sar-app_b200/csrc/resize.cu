@@ -294,6 +294,7 @@ constexpr int kMaxTileRadius = 6;          // of the row filter
 constexpr int kMaxTileColRadius = 15;      // of the column filter
 constexpr int kTileCols = 128;            // window columns, 256 / kTileCols row segments
 constexpr size_t kTileSmem = 48 * 1024;   // filtered rows
+constexpr int kMaxTileRows = 64, kMaxTileCols = 256;  // outputs of a tile
 
 // Extremes of a component as bits that order like the values, all from 0 on:
 // [0] ~min in, [1] max in, [2] ~min out, [3] max out, [4] NaN written.
@@ -550,11 +551,11 @@ bool tile_shape(const ResizePlan &p, const void *in, const void *out, int *orn, 
     const int r1 = std::max(p.radius[1], 0);
     const double c = (kTileCols - 3 - 2 * r1) / p.zoom[1];
     if (c < 8.0) return false;
-    *ocn = (int)std::min<double>({c, 256.0, (double)p.ocols});
+    *ocn = (int)std::min<double>({c, (double)kMaxTileCols, (double)p.ocols});
     const double wcols = std::min<double>(kTileCols, std::ceil(p.zoom[1] * *ocn) + 3 + 2 * r1);
     const double r = std::floor((double)kTileSmem / (wcols * p.nc * sizeof(T))) - 3;
     if (r < p.zoom[0]) return false;
-    *orn = (int)std::min<double>({r / p.zoom[0], 64.0, (double)p.orows});
+    *orn = (int)std::min<double>({r / p.zoom[0], (double)kMaxTileRows, (double)p.orows});
     return *orn >= 1;
 }
 
@@ -562,6 +563,10 @@ template <typename T, int NC>
 cudaError_t launch_tiles(const ResizePlan &p, const T *in, T *out, unsigned long long *stats, int orn, int ocn,
                          cudaStream_t st) {
     const long long tiles = (long long)((p.orows + orn - 1) / orn) * ((p.ocols + ocn - 1) / ocn);
+    // The kernel's limit belongs to the device, not to a context, so every call
+    // sets it to the most that any tile needs: a call's own size would refuse
+    // the launch of another thread's larger tile that comes just after it
+    constexpr int kSmemLimit = (int)(kTileSmem + (kMaxTileRows + kMaxTileCols) * sizeof(TileTap));
     const size_t smem = kTileSmem + (size_t)(orn + ocn) * sizeof(TileTap);
     cudaError_t e = cudaMemsetAsync(stats, 0, NC * kStatWords * sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
@@ -571,7 +576,7 @@ cudaError_t launch_tiles(const ResizePlan &p, const T *in, T *out, unsigned long
     switch (p.radius[0]) {
 #define X(R)                                                                                                        \
     case R:                                                                                                         \
-        e = cudaFuncSetAttribute(resize_tile_kernel<T, NC, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        e = cudaFuncSetAttribute(resize_tile_kernel<T, NC, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit); \
         if (e != cudaSuccess) return e;                                                                             \
         resize_tile_kernel<T, NC, R><<<(unsigned)tiles, 256, smem, st>>>(in, out, p.rows, p.cols, p.orows, p.ocols,  \
                                                                          p.zoom[0], p.zoom[1], w, p.radius[1], orn,  \

@@ -135,3 +135,28 @@ def test_tile_kernel_clips_like_the_steps(ctx, dtype, shape_out):
         got, want = _device(ctx, torch, b, shape_out), _device(ctx, torch, b, shape_out, shift=1)
         tol = (1e-6 if dtype == np.float32 else 1e-14) * 5
         np.testing.assert_allclose(got, want, rtol=0, atol=tol)
+
+
+def test_contexts_on_several_threads_resize_different_shapes(sb):
+    """Shapes whose tiles need different amounts of shared memory from the same
+    kernel, each from a context and a thread of its own."""
+    import threading
+
+    import torch
+    jobs = [((80, 70, 2), (640, 700)), ((9, 7, 2), (12, 10)), ((5, 40, 2), (7, 90))]
+    errors = []
+
+    def work(shape_in, shape_out):
+        try:
+            a = np.random.default_rng(4).normal(size=shape_in)
+            with sb.Context(0) as c:
+                first = _device(c, torch, a, shape_out)
+                for _ in range(400):
+                    assert np.array_equal(_device(c, torch, a, shape_out), first)
+        except Exception as e:
+            errors.append(e)
+
+    ts = [threading.Thread(target=work, args=j) for j in jobs for _ in range(2)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    assert not errors, errors[:2]
