@@ -287,7 +287,10 @@ __global__ void __launch_bounds__(kThreads) bounds_final_kernel(const double *__
 // output.  The clip bounds need the whole input, so the CTAs collect the
 // extremes of what they read and of what they wrote, and clip_kernel goes over
 // the output only if something lies outside (values rounded past the extremes,
-// NaN).  A kernel per step moved the array through memory four times: 1999 x
+// NaN).  The filters' sums are written as the roundings of the step kernels'
+// loops (left to the compiler, the unrolled row filter merged the centre's
+// product instead of the first pair's, and values differed in the last place),
+// so both paths give the same values bit for bit.  A kernel per step moved the array through memory four times: 1999 x
 // 1800 complex128 to half 129 us, 59 us in one; to twice 129 -> 81
 // us; 2000 x 2000 to a quarter 192 -> 75 us.
 constexpr int kMaxTileRadius = 6;          // of the row filter
@@ -406,10 +409,10 @@ __global__ void __launch_bounds__(256, 3)
                 if (R0 >= 0) {
 #pragma unroll
                     for (int k = 0; k < NC; ++k) {
-                        double acc = (double)ring[RH].v[k] * wt[0];
+                        double acc = __dmul_rn((double)ring[RH].v[k], wt[0]);
 #pragma unroll
                         for (int t = RH; t >= 1; --t)
-                            acc += ((double)ring[RH - t].v[k] + (double)ring[RH + t].v[k]) * wt[t];
+                            acc = __fma_rn((double)ring[RH - t].v[k] + (double)ring[RH + t].v[k], wt[t], acc);
                         f.v[k] = (T)acc;
                     }
                 }
@@ -431,12 +434,12 @@ __global__ void __launch_bounds__(256, 3)
                 if (c < ncol - 2 * r1h) {
                     double acc[NC];
 #pragma unroll
-                    for (int k = 0; k < NC; ++k) acc[k] = (double)row[c].v[k] * w.w1[0];
+                    for (int k = 0; k < NC; ++k) acc[k] = __dmul_rn((double)row[c].v[k], w.w1[0]);
                     for (int t = r1; t >= 1; --t) {
                         const E m = row[c - t], n = row[c + t];
                         const double wt = w.w1[t];
 #pragma unroll
-                        for (int k = 0; k < NC; ++k) acc[k] += ((double)m.v[k] + (double)n.v[k]) * wt;
+                        for (int k = 0; k < NC; ++k) acc[k] = __fma_rn((double)m.v[k] + (double)n.v[k], wt, acc[k]);
                     }
 #pragma unroll
                     for (int k = 0; k < NC; ++k) f[q].v[k] = (T)acc[k];

@@ -160,3 +160,19 @@ def test_contexts_on_several_threads_resize_different_shapes(sb):
     [t.start() for t in ts]
     [t.join() for t in ts]
     assert not errors, errors[:2]
+
+
+@pytest.mark.parametrize("shape_in,shape_out", [((300, 260), (150, 130)), ((131, 129), (40, 37)), ((90, 90), (89, 91)),
+                                                ((64, 300), (64, 80)), ((70, 33), (200, 115))])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("nc", [1, 2])
+def test_tile_kernel_rounds_like_the_steps(ctx, shape_in, shape_out, dtype, nc):
+    import torch
+    a = np.random.default_rng(12).normal(size=shape_in + (nc,)).astype(dtype)
+    # an output off its elements' alignment is formed step by step
+    if nc == 2:
+        want = _device(ctx, torch, a, shape_out, shift=1)
+    else:
+        three = np.repeat(a, 3, axis=2)
+        want = _device(ctx, torch, three, shape_out)[..., :1]
+    assert np.array_equal(_device(ctx, torch, a, shape_out), want)
