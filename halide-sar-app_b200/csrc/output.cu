@@ -62,7 +62,9 @@ __device__ __forceinline__ uint8_t u8_of(double2 z, const U8Scale &u) {
     const float a = (float)a2, x = a * u.inv_m2;
     const float q = fmaf(u.k, logf(x), u.q0);
     const float f = q - floorf(q);
-    if (a >= FLT_MIN && a <= FLT_MAX && x >= FLT_MIN) {  // (an f32 overflow or underflow says nothing)
+    // an f32 underflow says nothing (nothing overflows: |z| <= m, and m^2 is
+    // at most 1 / FLT_MIN unless eps is infinite)
+    if (a >= FLT_MIN && x >= FLT_MIN) {
         if (q > u.eps && q < 255.0f - u.eps && f > u.eps && f < 1.0f - u.eps) return (uint8_t)q;
         if (q < -u.eps) return 0;
         if (q > 255.0f + u.eps) return 255;
