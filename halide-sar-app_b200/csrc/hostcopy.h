@@ -11,46 +11,55 @@
 #include <cuda_runtime.h>
 #include <sys/types.h>
 
-#include <cstddef>
+#include <atomic>
+#include <condition_variable>
+#include <deque>
+#include <mutex>
+#include <thread>
+#include <vector>
 
 namespace sarbp {
 
-// Threads that share one memcpy at a time with the caller.  They start with
-// the first copy of several pieces, spin for the next copy for a short while
-// and then sleep.
+// Threads that share one memcpy at a time with the caller.  They wait on a
+// condition variable between sessions and spin within one (begin .. end).
 class CopyThreads {
 public:
-    CopyThreads() = default;
-    CopyThreads(const CopyThreads &) = delete;
     ~CopyThreads();
+    void begin();
+    void end();
     void copy(char *dst, const char *src, size_t n);
-    // No copy follows soon: spinning threads sleep at once.
-    void rest();
 
 private:
-    // Threads, lock and condition variable of the process that started them.
-    // A forked child has none of the threads, and the lock and the condition
-    // variable as the fork found them, so there it is left alone and never
-    // freed, and the caller copies by itself.
-    struct State;
-    State *state();
-    State *s_ = nullptr;
+    void work();
+    bool take(unsigned gen);
+    static constexpr size_t kPiece = 128 << 10;
+    std::vector<std::thread> threads_;
+    std::mutex mu_;
+    std::condition_variable cv_;
+    bool started_ = false, stop_ = false;
+    std::atomic<bool> session_{false};
+    // the copy in hand: generation in the high half, next piece in the low one
+    std::atomic<unsigned long long> next_{0};
+    std::atomic<unsigned> left_{0};  // pieces not yet done
+    std::atomic<unsigned> npieces_{0};
+    char *dst_ = nullptr;
+    const char *src_ = nullptr;
+    size_t n_ = 0;
+    unsigned gen_ = 0;
     pid_t pid_ = 0;
-    bool tried_ = false;
 };
 
 class HostStager {
 public:
     // Whether staging pays for a copy of n bytes at p (pageable, not small).
     static bool wants(const void *p, size_t n);
-    // One session per host-buffer call; its end drops what a failed call left
-    // in the slots and lets the threads sleep.
+    // One session per host-buffer call; the destructor ends it.
     class Session {
     public:
-        explicit Session(HostStager *s) : s_(s) {}
+        explicit Session(HostStager *s) : s_(s) { s_->threads_.begin(); }
         ~Session() {
             s_->abandon();
-            s_->threads_.rest();
+            s_->threads_.end();
         }
         Session(const Session &) = delete;
 
