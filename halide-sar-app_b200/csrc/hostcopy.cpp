@@ -4,12 +4,20 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <atomic>
+#include <condition_variable>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
+#include <new>
+#include <thread>
+#include <vector>
 
 namespace sarbp {
 
 namespace {
+constexpr size_t kPiece = 128 << 10;
+
 // One turn of a wait: a pause at first, then the core goes to whoever else
 // wants it (other contexts' threads, or a copying thread that lost its core).
 inline void relax(int turn) {
@@ -23,99 +31,117 @@ inline void relax(int turn) {
 }
 }  // namespace
 
-CopyThreads::~CopyThreads() {
-    if (started_ && pid_ != getpid()) {  // a forked child has no such threads to join
-        new std::vector<std::thread>(std::move(threads_));
-        return;
-    }
-    {
-        std::lock_guard<std::mutex> lk(mu_);
-        stop_ = true;
-        session_.store(false);
-    }
-    cv_.notify_all();
-    for (std::thread &t : threads_) t.join();
-}
+struct CopyThreads::State {
+    std::vector<std::thread> threads;
+    std::mutex mu;
+    std::condition_variable cv;
+    bool stop = false;
+    std::atomic<bool> session{false};
+    // the copy in hand: generation in the high half, next piece in the low one
+    std::atomic<unsigned long long> next{0};
+    std::atomic<unsigned> left{0};  // pieces not yet done
+    std::atomic<unsigned> npieces{0};
+    char *dst = nullptr;
+    const char *src = nullptr;
+    size_t n = 0;
+    unsigned gen = 0;
 
-void CopyThreads::begin() {
-    if (!started_) {
-        started_ = true;
-        pid_ = getpid();
-        // half of the cores at most, the caller among them (16 cores: 1.33 ms with 3
-        // helpers, 1.23 with 5, 1.18 with 7)
-        const int n = std::min(7, (int)std::thread::hardware_concurrency() / 2 - 1);
-        for (int i = 0; i < n; ++i) {
-            try {
-                threads_.emplace_back(&CopyThreads::work, this);
-            } catch (...) {  // no more threads: fewer share the copies
-                break;
+    bool available() const { return (unsigned)next.load() < npieces.load(); }
+
+    // Takes and copies pieces until none is left.  A copy that has begun
+    // meanwhile fails the exchange, so dst, src and n are those of the piece's
+    // copy until its last piece is done.
+    void take() {
+        for (;;) {
+            unsigned long long v = next.load(std::memory_order_acquire);
+            const unsigned i = (unsigned)v;
+            if (i >= npieces.load(std::memory_order_acquire)) return;
+            if (!next.compare_exchange_weak(v, v + 1, std::memory_order_acq_rel)) continue;
+            const size_t o = (size_t)i * kPiece;
+            std::memcpy(dst + o, src + o, std::min(kPiece, n - o));
+            left.fetch_sub(1, std::memory_order_release);
+        }
+    }
+
+    void work() {
+        for (;;) {
+            {
+                std::unique_lock<std::mutex> lk(mu);
+                cv.wait(lk, [&] { return stop || session.load(); });
+                if (stop) return;
+            }
+            for (int k = 0; session.load(std::memory_order_relaxed); k += k < 4096) {
+                if (available()) {
+                    take();
+                    k = 0;
+                }
+                relax(k);
             }
         }
     }
-    if (threads_.empty()) return;
+};
+
+CopyThreads::~CopyThreads() {
+    if (!s_ || pid_ != getpid()) return;
     {
-        std::lock_guard<std::mutex> lk(mu_);
-        session_.store(true);
+        std::lock_guard<std::mutex> lk(s_->mu);
+        s_->stop = true;
+        s_->session.store(false);
     }
-    cv_.notify_all();
+    s_->cv.notify_all();
+    for (std::thread &t : s_->threads) t.join();
+    delete s_;
+}
+
+// The threads' state, or null where the caller copies alone.
+CopyThreads::State *CopyThreads::state() {
+    if (!tried_) {
+        tried_ = true;
+        // half of the cores at most, the caller among them (16 cores: 1.33 ms with 3
+        // helpers, 1.23 with 5, 1.18 with 7)
+        const int n = std::min(7, (int)std::thread::hardware_concurrency() / 2 - 1);
+        if (n < 1 || !(s_ = new (std::nothrow) State)) return nullptr;
+        pid_ = getpid();
+        try {
+            for (int i = 0; i < n; ++i) s_->threads.emplace_back(&State::work, s_);
+        } catch (...) {  // no more threads: fewer share the copies
+        }
+    }
+    return s_ && pid_ == getpid() && !s_->threads.empty() ? s_ : nullptr;
+}
+
+void CopyThreads::begin() {
+    State *s = state();
+    if (!s) return;
+    {
+        std::lock_guard<std::mutex> lk(s->mu);
+        s->session.store(true);
+    }
+    s->cv.notify_all();
 }
 
 void CopyThreads::end() {
-    if (!threads_.empty()) session_.store(false);
-}
-
-// Takes and copies pieces of generation gen until none is left.
-bool CopyThreads::take(unsigned gen) {
-    bool any = false;
-    for (;;) {
-        unsigned long long v = next_.load(std::memory_order_acquire);
-        if ((unsigned)(v >> 32) != gen) return any;
-        const unsigned i = (unsigned)v;
-        if (i >= npieces_.load(std::memory_order_acquire)) return any;
-        // (a changed generation fails the exchange, so dst_, src_ and n_ are
-        // those of this copy until its last piece is done)
-        if (!next_.compare_exchange_weak(v, v + 1, std::memory_order_acq_rel)) continue;
-        const size_t o = (size_t)i * kPiece;
-        std::memcpy(dst_ + o, src_ + o, std::min(kPiece, n_ - o));
-        left_.fetch_sub(1, std::memory_order_release);
-        any = true;
-    }
-}
-
-void CopyThreads::work() {
-    for (;;) {
-        {
-            std::unique_lock<std::mutex> lk(mu_);
-            cv_.wait(lk, [&] { return stop_ || session_.load(); });
-            if (stop_) return;
-        }
-        int idle = 0;
-        while (session_.load(std::memory_order_relaxed)) {
-            if (take((unsigned)(next_.load(std::memory_order_acquire) >> 32))) idle = 0;
-            for (int k = 0; k < 32 && idle < 4096; ++k) relax(idle++);
-            if (idle >= 4096) relax(idle);
-        }
-    }
+    if (s_ && pid_ == getpid()) s_->session.store(false);
 }
 
 void CopyThreads::copy(char *dst, const char *src, size_t n) {
     const size_t pieces = (n + kPiece - 1) / kPiece;
-    if (threads_.empty() || pieces < 2) {
+    State *s = pieces < 2 ? nullptr : state();
+    if (!s) {
         std::memcpy(dst, src, n);
         return;
     }
-    // no thread holds a piece here: the copy before ended with left_ == 0, and a
-    // thread that still looks at its generation finds no piece left
-    dst_ = dst;
-    src_ = src;
-    n_ = n;
-    left_.store((unsigned)pieces, std::memory_order_relaxed);
-    ++gen_;
-    next_.store((unsigned long long)gen_ << 32 | 0xffffffffull, std::memory_order_relaxed);  // none yet
-    npieces_.store((unsigned)pieces, std::memory_order_release);
-    next_.store((unsigned long long)gen_ << 32, std::memory_order_release);
-    take(gen_);
-    for (int k = 0; left_.load(std::memory_order_acquire) != 0; k += k < 4096) relax(k);
+    // no thread holds a piece here: the copy before ended with left == 0
+    s->left.store((unsigned)pieces, std::memory_order_relaxed);
+    ++s->gen;
+    s->next.store((unsigned long long)s->gen << 32 | 0xffffffffull);  // none yet
+    s->dst = dst;
+    s->src = src;
+    s->n = n;
+    s->npieces.store((unsigned)pieces);
+    s->next.store((unsigned long long)s->gen << 32);
+    s->take();
+    for (int k = 0; s->left.load(std::memory_order_acquire) != 0; k += k < 4096) relax(k);
 }
 
 bool HostStager::wants(const void *p, size_t n) {

@@ -11,12 +11,7 @@
 #include <cuda_runtime.h>
 #include <sys/types.h>
 
-#include <atomic>
-#include <condition_variable>
-#include <deque>
-#include <mutex>
-#include <thread>
-#include <vector>
+#include <cstddef>
 
 namespace sarbp {
 
@@ -24,29 +19,23 @@ namespace sarbp {
 // condition variable between sessions and spin within one (begin .. end).
 class CopyThreads {
 public:
+    CopyThreads() = default;
+    CopyThreads(const CopyThreads &) = delete;
     ~CopyThreads();
     void begin();
     void end();
     void copy(char *dst, const char *src, size_t n);
 
 private:
-    void work();
-    bool take(unsigned gen);
-    static constexpr size_t kPiece = 128 << 10;
-    std::vector<std::thread> threads_;
-    std::mutex mu_;
-    std::condition_variable cv_;
-    bool started_ = false, stop_ = false;
-    std::atomic<bool> session_{false};
-    // the copy in hand: generation in the high half, next piece in the low one
-    std::atomic<unsigned long long> next_{0};
-    std::atomic<unsigned> left_{0};  // pieces not yet done
-    std::atomic<unsigned> npieces_{0};
-    char *dst_ = nullptr;
-    const char *src_ = nullptr;
-    size_t n_ = 0;
-    unsigned gen_ = 0;
+    // Threads, lock and condition variable of the process that started them.
+    // A forked child has none of the threads, and the lock and the condition
+    // variable as the fork found them, so there it is left alone and never
+    // freed, and the caller copies by itself.
+    struct State;
+    State *state();
+    State *s_ = nullptr;
     pid_t pid_ = 0;
+    bool tried_ = false;
 };
 
 class HostStager {
