@@ -15,16 +15,17 @@
 
 namespace sarbp {
 
-// Threads that share one memcpy at a time with the caller.  They wait on a
-// condition variable between sessions and spin within one (begin .. end).
+// Threads that share one memcpy at a time with the caller.  They start with
+// the first copy of several pieces, spin for the next copy for a short while
+// and then sleep.
 class CopyThreads {
 public:
     CopyThreads() = default;
     CopyThreads(const CopyThreads &) = delete;
     ~CopyThreads();
-    void begin();
-    void end();
     void copy(char *dst, const char *src, size_t n);
+    // No copy follows soon: spinning threads sleep at once.
+    void rest();
 
 private:
     // Threads, lock and condition variable of the process that started them.
@@ -42,13 +43,14 @@ class HostStager {
 public:
     // Whether staging pays for a copy of n bytes at p (pageable, not small).
     static bool wants(const void *p, size_t n);
-    // One session per host-buffer call; the destructor ends it.
+    // One session per host-buffer call; its end drops what a failed call left
+    // in the slots and lets the threads sleep.
     class Session {
     public:
-        explicit Session(HostStager *s) : s_(s) { s_->threads_.begin(); }
+        explicit Session(HostStager *s) : s_(s) {}
         ~Session() {
             s_->abandon();
-            s_->threads_.end();
+            s_->threads_.rest();
         }
         Session(const Session &) = delete;
 

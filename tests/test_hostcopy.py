@@ -9,9 +9,11 @@ import pytest
 from conftest import PKG
 
 HARNESS = r"""
+#include <dirent.h>
 #include <signal.h>
 #include <stdlib.h>
 #include <string.h>
+#include <sys/resource.h>
 #include <sys/wait.h>
 #include <unistd.h>
 #include <cstdio>
@@ -41,6 +43,18 @@ cudaError_t cudaFreeHost(void *p) { free(p); return cudaSuccess; }
 
 using sarbp::HostStager;
 
+static int threads() {
+    int n = 0;
+    DIR *d = opendir("/proc/self/task");
+    while (dirent *e = readdir(d)) n += e->d_name[0] != '.';
+    closedir(d);
+    return n;
+}
+static double cpu_seconds() {
+    rusage r;
+    getrusage(RUSAGE_SELF, &r);
+    return r.ru_utime.tv_sec + r.ru_stime.tv_sec + 1e-6 * (r.ru_utime.tv_usec + r.ru_stime.tv_usec);
+}
 // n bytes up and down again; whether they arrived
 static bool round_trip(HostStager &s, size_t n, unsigned seed) {
     std::vector<char> a(n), dev(n), b(n);
@@ -59,6 +73,17 @@ int main(int, char **argv) {
         const size_t sizes[] = {1, 128 << 10, (128 << 10) + 1, (2 << 20) - 1, 2 << 20, (2 << 20) + 4097, 40000003};
         for (int rep = 0; rep < 20; ++rep)
             for (size_t n : sizes) ok = ok && round_trip(*s, rep < 10 || n < (3 << 20) ? n : 1000, rep);
+    } else if (!strcmp(argv[1], "nothing_staged")) {
+        HostStager::Session session(s);
+        ok = threads() == 1;
+    } else if (!strcmp(argv[1], "idle")) {
+        std::vector<char> a(8 << 20, 1), dev(8 << 20);
+        HostStager::Session session(s);
+        ok = s->upload(dev.data(), a.data(), a.size(), nullptr) == cudaSuccess;
+        const double t = cpu_seconds();
+        usleep(500000);  // a kernel runs
+        ok = ok && cpu_seconds() - t < 0.1;
+        ok = ok && round_trip(*s, 9000001, 5);
     } else if (!strcmp(argv[1], "fork")) {
         ok = round_trip(*s, 9000001, 1);
         usleep(100000);  // the threads sleep
@@ -99,8 +124,10 @@ def exe(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("what", ["data", "fork"])
+@pytest.mark.parametrize("what", ["data", "fork", "nothing_staged", "idle"])
 def test_staged_copies(exe, what):
-    """The bytes arrive; a forked child copies by itself and may drop the object."""
+    """The bytes arrive; a forked child copies by itself and may drop the
+    object; threads start with the first staged copy and sleep while nothing is
+    copied."""
     p = subprocess.run([exe, what], capture_output=True, text=True, timeout=120)
     assert p.returncode == 0 and p.stdout.strip() == "ok", p.stdout
