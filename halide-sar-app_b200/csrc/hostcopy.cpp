@@ -170,13 +170,20 @@ cudaError_t HostStager::settle(Slot &s, int i) {
     return cudaSuccess;
 }
 
+// The slots; false where there is no page-locked memory to be had.
+bool HostStager::ready() {
+    if (pin_) return true;
+    void *p = nullptr;
+    if (cudaMallocHost(&p, kSlotBytes * kSlots) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    pin_ = static_cast<char *>(p);
+    return true;
+}
+
 cudaError_t HostStager::acquire(int *slot) {
     cudaError_t e = cudaSuccess;
-    if (!pin_) {
-        void *p = nullptr;
-        if ((e = cudaMallocHost(&p, kSlotBytes * kSlots)) != cudaSuccess) return e;
-        pin_ = static_cast<char *>(p);
-    }
     Slot &s = slots_[next_];
     if (!s.ev && (e = cudaEventCreateWithFlags(&s.ev, cudaEventDisableTiming)) != cudaSuccess) return e;
     if ((e = settle(s, next_)) != cudaSuccess) return e;
@@ -186,6 +193,7 @@ cudaError_t HostStager::acquire(int *slot) {
 }
 
 cudaError_t HostStager::upload(void *dst, const void *src, size_t n, cudaStream_t st) {
+    if (!ready()) return cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, st);
     for (size_t o = 0; o < n; o += kSlotBytes) {
         const size_t m = std::min(kSlotBytes, n - o);
         int i = 0;
@@ -202,6 +210,7 @@ cudaError_t HostStager::upload(void *dst, const void *src, size_t n, cudaStream_
 }
 
 cudaError_t HostStager::download(void *dst, const void *src, size_t n, cudaStream_t st) {
+    if (!ready()) return cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, st);
     for (size_t o = 0; o < n; o += kSlotBytes) {
         const size_t m = std::min(kSlotBytes, n - o);
         int i = 0;

@@ -60,6 +60,7 @@ public:
     // dst (device) <- src (host) on st; src has been read when this returns.
     cudaError_t upload(void *dst, const void *src, size_t n, cudaStream_t st);
     // dst (host) <- src (device) behind what st holds; complete after drain().
+    // Both copy directly where no page-locked memory is to be had.
     cudaError_t download(void *dst, const void *src, size_t n, cudaStream_t st);
     cudaError_t drain();
     // Waits for the copies in flight and frees the slots.
@@ -74,6 +75,7 @@ private:
         char *out = nullptr;  // destination of a download still in the slot
         size_t n = 0;
     };
+    bool ready();
     cudaError_t acquire(int *slot);
     cudaError_t settle(Slot &s, int i);
     void abandon();  // drops downloads that a failed call left behind

@@ -20,6 +20,7 @@ HARNESS = r"""
 #include <vector>
 #include "hostcopy.h"
 
+static bool g_no_pin = false;
 extern "C" {
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) {
     memset(a, 0, sizeof(*a));
@@ -36,9 +37,12 @@ cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cu
     return cudaSuccess;
 }
 cudaError_t cudaMallocHost(void **p, size_t n) {
+    if (g_no_pin) return cudaErrorMemoryAllocation;
     return (*p = malloc(n)) ? cudaSuccess : cudaErrorMemoryAllocation;
 }
 cudaError_t cudaFreeHost(void *p) { free(p); return cudaSuccess; }
+cudaError_t cudaHostRegister(void *, size_t, unsigned) { return g_no_pin ? cudaErrorMemoryAllocation : cudaSuccess; }
+cudaError_t cudaHostUnregister(void *) { return cudaSuccess; }
 }
 
 using sarbp::HostStager;
@@ -102,6 +106,11 @@ int main(int, char **argv) {
             return 1;
         }
         ok = ok && WIFEXITED(st) && WEXITSTATUS(st) == 0 && round_trip(*s, 9000001, 3);
+    } else if (!strcmp(argv[1], "no_page_locked_memory")) {
+        g_no_pin = true;
+        ok = round_trip(*s, 9000001, 4);
+        g_no_pin = false;
+        ok = ok && round_trip(*s, 9000001, 5);
     }
     s->release();
     delete s;
@@ -124,10 +133,10 @@ def exe(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("what", ["data", "fork", "nothing_staged", "idle"])
+@pytest.mark.parametrize("what", ["data", "fork", "nothing_staged", "idle", "no_page_locked_memory"])
 def test_staged_copies(exe, what):
     """The bytes arrive; a forked child copies by itself and may drop the
     object; threads start with the first staged copy and sleep while nothing is
-    copied."""
+    copied; without page-locked memory the copies are the driver's."""
     p = subprocess.run([exe, what], capture_output=True, text=True, timeout=120)
     assert p.returncode == 0 and p.stdout.strip() == "ok", p.stdout
