@@ -1,6 +1,7 @@
 // hostcopy.cpp -- see hostcopy.h.
 #include "hostcopy.h"
 
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include <algorithm>
@@ -49,8 +50,8 @@ struct CopyThreads::State {
     std::atomic<unsigned> left{0};  // pieces not yet done
     std::atomic<unsigned> npieces{0};
     char *dst = nullptr;
-    const char *src = nullptr;
-    size_t n = 0;
+    const char *src = nullptr;  // null: zeros
+    size_t n = 0, piece = 0;
     unsigned gen = 0;
 
     bool available() const { return (unsigned)next.load() < npieces.load(); }
@@ -64,8 +65,11 @@ struct CopyThreads::State {
             const unsigned i = (unsigned)v;
             if (i >= npieces.load(std::memory_order_acquire)) return;
             if (!next.compare_exchange_weak(v, v + 1, std::memory_order_acq_rel)) continue;
-            const size_t o = (size_t)i * kPiece;
-            std::memcpy(dst + o, src + o, std::min(kPiece, n - o));
+            const size_t o = (size_t)i * piece, m = std::min(piece, n - o);
+            if (src)
+                std::memcpy(dst + o, src + o, m);
+            else
+                std::memset(dst + o, 0, m);
             left.fetch_sub(1, std::memory_order_release);
         }
     }
@@ -123,11 +127,18 @@ void CopyThreads::rest() {
     if (s_ && pid_ == getpid()) s_->active.store(false);
 }
 
-void CopyThreads::copy(char *dst, const char *src, size_t n) {
-    const size_t pieces = (n + kPiece - 1) / kPiece;
+void CopyThreads::copy(char *dst, const char *src, size_t n) { run(dst, src, n, kPiece); }
+
+void CopyThreads::zero(char *dst, size_t n, size_t piece) { run(dst, nullptr, n, piece); }
+
+void CopyThreads::run(char *dst, const char *src, size_t n, size_t piece) {
+    const size_t pieces = (n + piece - 1) / piece;
     State *s = pieces < 2 ? nullptr : state();
     if (!s) {
-        std::memcpy(dst, src, n);
+        if (src)
+            std::memcpy(dst, src, n);
+        else
+            std::memset(dst, 0, n);
         return;
     }
     s->active.store(true);
@@ -138,6 +149,7 @@ void CopyThreads::copy(char *dst, const char *src, size_t n) {
     s->dst = dst;
     s->src = src;
     s->n = n;
+    s->piece = piece;
     s->npieces.store((unsigned)pieces);
     s->next.store((unsigned long long)s->gen << 32);
     // a thread counts itself as sleeping before it looks for pieces a last time
@@ -170,15 +182,28 @@ cudaError_t HostStager::settle(Slot &s, int i) {
     return cudaSuccess;
 }
 
-// The slots; false where there is no page-locked memory to be had.
+// The slots; false where there is no page-locked memory to be had.  A
+// context's first call waits for the locking of 16 MB, so they are mapped in
+// huge pages where the system has them and the threads touch the pages ahead
+// of it: 1.2 ms, against 2.9 without the threads and 8 with cudaMallocHost
+// (the first 768^2 x 800 call of a context 6 ms, as with the driver's own
+// staging, against 8 and 20).
 bool HostStager::ready() {
     if (pin_) return true;
-    void *p = nullptr;
-    if (cudaMallocHost(&p, kSlotBytes * kSlots) != cudaSuccess) {
+    constexpr size_t kHuge = 2 << 20, kBytes = kSlotBytes * kSlots;
+    void *p = mmap(nullptr, kBytes + kHuge, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (p == MAP_FAILED) return false;
+    char *at = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(p) + kHuge - 1) / kHuge * kHuge);
+    madvise(at, kBytes, MADV_HUGEPAGE);
+    threads_.zero(at, kBytes, kHuge);  // a page a thread, ahead of the locking
+    if (cudaHostRegister(at, kBytes, cudaHostRegisterPortable) != cudaSuccess) {
         cudaGetLastError();
+        munmap(p, kBytes + kHuge);
         return false;
     }
-    pin_ = static_cast<char *>(p);
+    map_ = p;
+    map_bytes_ = kBytes + kHuge;
+    pin_ = at;
     return true;
 }
 
@@ -252,7 +277,10 @@ void HostStager::release() {
         if (s.ev) cudaEventDestroy(s.ev);
         s = Slot{};
     }
-    if (pin_) cudaFreeHost(pin_);
+    if (pin_) {
+        cudaHostUnregister(pin_);
+        munmap(map_, map_bytes_);
+    }
     pin_ = nullptr;
 }
 

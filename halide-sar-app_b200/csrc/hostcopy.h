@@ -24,6 +24,7 @@ public:
     CopyThreads(const CopyThreads &) = delete;
     ~CopyThreads();
     void copy(char *dst, const char *src, size_t n);
+    void zero(char *dst, size_t n, size_t piece);  // a piece to a thread
     // No copy follows soon: spinning threads sleep at once.
     void rest();
 
@@ -34,6 +35,7 @@ private:
     // freed, and the caller copies by itself.
     struct State;
     State *state();
+    void run(char *dst, const char *src, size_t n, size_t piece);
     State *s_ = nullptr;
     pid_t pid_ = 0;
     bool tried_ = false;
@@ -81,6 +83,8 @@ private:
     void abandon();  // drops downloads that a failed call left behind
     CopyThreads threads_;
     char *pin_ = nullptr;
+    void *map_ = nullptr;  // the mapping that holds pin_
+    size_t map_bytes_ = 0;
     Slot slots_[kSlots];
     int next_ = 0;
 };
