@@ -431,8 +431,8 @@ __device__ __forceinline__ bool stage_windows(const DevJob &jb, int lane, int p0
 }
 
 // Launch counters, zero before the launch: [0] items claimed beyond the first
-// of each CTA, [1] SMs that run CTAs of the launch, [2] CTAs started, then
-// from word 4 what the CTAs of each SM took: items, one byte per SM
+// of each CTA, [1] SMs that run CTAs of the launch, [2] CTAs started,
+// [kBpZeroWord] nothing, then from word 4 what the CTAs of each SM took: items, one byte per SM
 // (kDealItems), or pulses, one word per SM (kDealPulses).
 struct Claims {
     int *ctr;

@@ -71,7 +71,8 @@ size_t bp_smem_bytes(const BpLaunch &L);
 int bp_max_active_blocks(const BpLaunch &L);
 cudaError_t init_backproject_attributes();
 // d_counter: kBpCounterBytes of device memory (kBpDealBytes with kDealPulses),
-// zero before a persistent launch
+// zero before a persistent launch; word kBpZeroWord stays zero
+constexpr int kBpZeroWord = 3;
 constexpr int kBpCounterBytes = 256, kBpDealSms = 252, kBpDealBytes = 16 + 4 * kBpDealSms;
 cudaError_t launch_backproject(const BpLaunch &L, const DevJob *d_jobs, const WorkItem *d_items,
                                int nitems, int *d_counter, cudaStream_t st);

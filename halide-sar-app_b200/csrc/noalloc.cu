@@ -236,8 +236,16 @@ extern "C" int sarbp_backprojection_noalloc(const sarbp_job *job, void *cuda_str
     dj.out_u8 = j.out_u8;
     dj.dB_min = j.dB_min;
     dj.dB_max = j.dB_max;
+    BpLaunch L = L0;
+    const int occ = bp_max_active_blocks(L);
+    if (occ < 1) return fail(SARBP_ERR_CUDA, "no-alloc: backprojection kernel does not fit on an SM");
+    L.grid = (int)std::min<long long>((long long)occ * num_sms, (long long)nitems);
+    L.deal.how = kDealItems;  // one job: its parts differ by a pulse at most
     dj.nsplit = nsplit;
-    dj.sum_parts = 1;
+    // a tile's parts are added by its last item where every CTA has one item, by
+    // the combine kernel in longer lists (400^2 x 900: 176 us a call in place,
+    // 154 so)
+    dj.sum_parts = nitems <= (size_t)L.grid;
     dj.parts = nsplit > 1 ? reinterpret_cast<float2 *>(sb + o_parts) : nullptr;
 
     DevJob *d_job = reinterpret_cast<DevJob *>(sb + o_job);
@@ -253,12 +261,10 @@ extern "C" int sarbp_backprojection_noalloc(const sarbp_job *job, void *cuda_str
     e = launch_range_compress(logN, d_job, d_rows, j.npulses, 1, d_tw, st);
     if (e == cudaSuccess) e = launch_tile_setup(d_job, d_items, (int)ntiles, L0.tile_x * L0.tile_y, st);
     if (e != cudaSuccess) return cuda_fail(e, "no-alloc range compression / geometry launch");
-    BpLaunch L = L0;
-    const int occ = bp_max_active_blocks(L);
-    if (occ < 1) return fail(SARBP_ERR_CUDA, "no-alloc: backprojection kernel does not fit on an SM");
-    L.grid = (int)std::min<long long>((long long)occ * num_sms, (long long)nitems);
-    L.deal.how = kDealItems;  // one job: its parts differ by a pulse at most
     e = launch_backproject(L, d_job, d_items, (int)nitems, d_cnt, st);
+    // (the combine kernel's list of jobs, {0}, is the word that the counters leave unused)
+    if (e == cudaSuccess && nsplit > 1 && !dj.sum_parts)
+        e = launch_combine_parts(d_job, d_cnt + kBpZeroWord, 1, (long long)j.nu * j.nv, num_sms, st);
     if (e == cudaSuccess && j.out_u8) e = launch_batch_u8(d_job, 1, u8_chunks((long long)j.nu * j.nv), st);
     if (e == cudaSuccess && status) {
         status_kernel<<<1, 1, 0, st>>>(dj.sc, status);

@@ -539,7 +539,7 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
     const size_t o_comb = align_up(o_tiles + tiles.size() * sizeof(WorkItem), 256);
     const size_t o_cnt = align_up(o_comb + combine.size() * sizeof(int), 256);
     const size_t cnt_bytes = slabs ? kBpCounterBytes * (size_t)slabs->nslabs : (size_t)kBpDealBytes;
-    const size_t meta_bytes = o_cnt + cnt_bytes + sizeof(int);
+    const size_t meta_bytes = o_cnt + cnt_bytes;
     if (for_graph && ((!single && host_meta_.cap < meta_bytes) || meta_.cap < meta_bytes))
         return fail(SARBP_ERR_STATE, "graph capture needs a prior run of the same jobs");
     if (!single) {
@@ -604,8 +604,8 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
     // (one job's items begin with part 0 of every tile)
     const WorkItem *d_tiles = single || !any_split ? d_items : reinterpret_cast<const WorkItem *>(d + o_tiles);
     int *d_cnt = reinterpret_cast<int *>(d + o_cnt);
-    // (one job's counters are followed by a zero: its index in the list)
-    const int *d_comb = single ? d_cnt + cnt_bytes / sizeof(int) : reinterpret_cast<const int *>(d + o_comb);
+    // (one job's list is {0}: the word that its counters leave unused)
+    const int *d_comb = single ? d_cnt + kBpZeroWord : reinterpret_cast<const int *>(d + o_comb);
 
     // twiddle tables first (a one-time synchronous upload per N_fft; a
     // four-step N_fft also needs the tables of its two sub-lengths)
@@ -625,7 +625,7 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
     if ((e = rec(0)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
     if (single) {
         e = launch_prep_single(one, SingleLists{d_jobs, d_items, (int)ntile_items, (int)nitems, d_rows,
-                                                (int)nrows_total, d_cnt, (int)(cnt_bytes / sizeof(int)) + 1}, st);
+                                                (int)nrows_total, d_cnt, (int)(cnt_bytes / sizeof(int))}, st);
         if (e != cudaSuccess) return cuda_fail(e, "set-up launch");
     } else {
         launch_prep(d_jobs, njobs, st);

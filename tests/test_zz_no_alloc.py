@@ -132,3 +132,24 @@ def test_noalloc_rejects_jobs_larger_than_its_scratch(sb):
     # N_fft above 16384 (the four-step FFT's work buffer) is not taken either
     job = sb.make_job(64, 8, 32768, 17, 32, 32, 0.25, 16, 16, 16, 16, r=16)
     assert L.sarbp_backprojection_noalloc(ctypes.byref(job), None, None) == _lib.ERR_UNSUPPORTED
+
+
+# one round of items with the parts' sum in place; several rounds and the combine kernel
+@pytest.mark.parametrize("n,P", [(256, 300), (400, 900), (330, 1111)])
+def test_noalloc_pulse_parts_equal_the_device_entry_point(sb, ctx, n, P):
+    import torch
+    from sarbp_b200 import _lib, synth
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    d = synth.make("plain_small", seed=5, with_r=True, overrides=dict(P=P, S=200, n=n, extent=25.0, taylor=20))
+    t = dict(phs=dev(d["phs"].view(np.float32)), k=dev(d["k_r"].astype(np.float32)),
+             pos=dev(d["pos"].astype(np.float32)), r=dev(d["r"]))
+    kw = dict(r=t["r"].data_ptr(), dB_min=-40.0, dB_max=0.0)
+    ref, ref_u8 = torch.zeros((n, n, 2), dtype=torch.float64, device="cuda"), torch.zeros((n, n), dtype=torch.uint8, device="cuda")
+    got, got_u8 = torch.full_like(ref, float("nan")), torch.zeros_like(ref_u8)
+    ctx.run_jobs([_job(sb, d, t, sb.PREC_COMPAT, kw, ref, ref_u8)])
+    ctx.synchronize()
+    job = _job(sb, d, t, sb.PREC_COMPAT, kw, got, got_u8)
+    for _ in range(2):
+        assert _lib.lib().sarbp_backprojection_noalloc(ctypes.byref(job), None, None) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(got, ref) and torch.equal(got_u8, ref_u8)
