@@ -559,7 +559,13 @@ bool tile_shape(const ResizePlan &p, const void *in, const void *out, int *orn, 
     const double r = std::floor((double)kTileSmem / (wcols * p.nc * sizeof(T))) - 3;
     if (r < p.zoom[0]) return false;
     *orn = (int)std::min<double>({r / p.zoom[0], (double)kMaxTileRows, (double)p.orows});
-    return *orn >= 1;
+    if (*orn < 1) return false;
+    auto ctas = [&] { return (long long)((p.orows + *orn - 1) / *orn) * ((p.ocols + *ocn - 1) / *ocn); };
+    // A few long rows leave most of a CTA idle, and its fixed cost (3.5 us a
+    // round of 444) is more than the steps' in many rounds: 1 x 1000000 f64
+    // to 400000 is 70 us in tiles and 38 in steps, 4 x 250000 to half 31 and 43
+    const long long n = std::max(p.rows, p.orows);
+    return n > 6 || n * (long long)elem > 48 || ctas() <= 1200 * (n + 1);
 }
 
 template <typename T, int NC>

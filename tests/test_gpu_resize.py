@@ -176,3 +176,16 @@ def test_tile_kernel_rounds_like_the_steps(ctx, shape_in, shape_out, dtype, nc):
         three = np.repeat(a, 3, axis=2)
         want = _device(ctx, torch, three, shape_out)[..., :1]
     assert np.array_equal(_device(ctx, torch, a, shape_out), want)
+
+
+# many tiles of few rows: beyond the line the steps, below it tiles
+@pytest.mark.parametrize("shape_in,shape_out", [((1, 600000), (1, 240000)), ((1, 100000), (1, 40000)),
+                                                ((3, 700001), (3, 350000)), ((4, 120000), (7, 240001))])
+@pytest.mark.parametrize("nc", [1, 2])
+def test_long_rows(ctx, shape_in, shape_out, nc):
+    import torch
+    from resize_oracle import sk_resize
+    a = np.random.default_rng(13).normal(size=shape_in + (nc,))
+    got = _device(ctx, torch, a, shape_out)
+    for k in range(nc):
+        _check(got[..., k], sk_resize(a[..., k], shape_out))
