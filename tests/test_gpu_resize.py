@@ -189,3 +189,13 @@ def test_long_rows(ctx, shape_in, shape_out, nc):
     got = _device(ctx, torch, a, shape_out)
     for k in range(nc):
         _check(got[..., k], sk_resize(a[..., k], shape_out))
+
+
+# few tiles, split by rows down to four
+@pytest.mark.parametrize("shape_in,shape_out", [((64, 64), (64, 1000)), ((9, 1000), (5, 400)), ((2000, 2), (1000, 2)),
+                                                ((300, 300), (77, 75)), ((3, 40), (2, 900)), ((469, 3), (301, 3))])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_split_tiles_round_like_the_steps(ctx, shape_in, shape_out, dtype):
+    import torch
+    a = np.random.default_rng(14).normal(size=shape_in + (2,)).astype(dtype)
+    assert np.array_equal(_device(ctx, torch, a, shape_out), _device(ctx, torch, a, shape_out, shift=1))
