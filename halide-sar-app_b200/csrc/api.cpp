@@ -111,7 +111,6 @@ int run_host_job(sarbp_ctx *ctx, const float *phs, int S, int P, const float *k_
     // pageable arrays go through page-locked slots (see hostcopy.h)
     const size_t n_out = npix * 2 * sizeof(double);
     const bool stage_r = r && HostStager::wants(r, npix * 3 * sizeof(double));
-    const bool stage_out = HostStager::wants(out, n_out);
     const HostStager::Session session(&ctx->stager);
     auto to_device = [&](void *dst, const void *src, size_t n, bool staged) {
         return staged ? ctx->stager.upload(dst, src, n, cin) : cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, cin);
@@ -127,16 +126,25 @@ int run_host_job(sarbp_ctx *ctx, const float *phs, int S, int P, const float *k_
         {d_u, r ? nullptr : plane->u, (size_t)nu * sizeof(double)},
         {d_v, r ? nullptr : plane->v, (size_t)nv * sizeof(double)},
     };
+    bool staged = stage_r;
     for (const Copy &c : copies) {
         if (!c.src) continue;
-        e = to_device(c.dst, c.src, c.n, HostStager::wants(c.src, c.n));
+        const bool stage = HostStager::wants(c.src, c.n);
+        staged = staged || stage;
+        e = to_device(c.dst, c.src, c.n, stage);
         if (e != cudaSuccess) return cuda_fail(e, "copying inputs to the device");
     }
+    // A small image is staged only where inputs were, so that the copy threads
+    // are awake: waking a thread holds the caller for up to 60 us, more than the
+    // driver's copy of a few MB takes longer (from page-locked arrays, 200^2 x 800:
+    // 430 us with the image staged, 227 with the driver's copy; 300^2 x 800: 603
+    // and 376; 700^2 x 800: 809 and 969)
+    const bool stage_out = (staged || n_out >= (4 << 20)) && HostStager::wants(out, n_out);
     SlabSpec spec;
     if (nslabs) {
-        spec.copy_stream = cin;  // descriptors after the phase history, before the positions
-        // the pixel positions go up slab by slab once the batch's descriptors
-        // and range compression are enqueued (see SlabSpec::before_slabs)
+        spec.copy_stream = cin;
+        // the pixel positions go up slab by slab once the set-up and the range
+        // compression are enqueued (see SlabSpec::before_slabs)
         spec.before_slabs = [&]() -> cudaError_t {
             for (int g = 0; g < nslabs && r; ++g) {
                 const size_t y0 = std::min((size_t)nv, (size_t)row0[g] * tile_y);

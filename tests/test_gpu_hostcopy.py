@@ -1,5 +1,6 @@
 """Host-buffer calls on pageable arrays (staged through page-locked slots by
 several threads) form the device call's image bit for bit; GPU tests."""
+import os
 import threading
 
 import numpy as np
@@ -78,3 +79,29 @@ def test_contexts_on_several_threads():
     with sb.Context(0) as c:
         for i in range(3):
             assert np.array_equal(_host(c, data[i], False), out[i])
+
+
+# page-locked inputs: none staged; the image is, from 4 MB on
+@pytest.mark.parametrize("nu,nv", [(100, 90), (300, 200), (500, 480), (640, 601)])
+def test_page_locked_arrays_equal_device_call(ctx, torch, nu, nv):
+    d = _data(nu, nv, 40, 64, seed=nu)
+    want = _device(ctx, torch, d, False)
+    pinned = {k: torch.from_numpy(np.ascontiguousarray(d[k], t)).pin_memory().numpy()
+              for k, t in (("k_r", np.float32), ("pos", np.float32), ("r", np.float64))}
+    phs = torch.from_numpy(np.ascontiguousarray(d["phs"], np.complex64).view(np.float32)).pin_memory().numpy()
+    for _ in range(3):
+        got = ctx.backprojection_cuda(phs.view(np.complex64), pinned["k_r"], 20, d["N_fft"], d["delta_r"], d["u"],
+                                      d["v"], pinned["pos"], pinned["r"])
+        assert np.array_equal(got, want)
+
+
+def test_a_small_image_alone_wakes_no_copy_threads(torch):
+    """Waking them takes longer than the driver's copy."""
+    d = _data(300, 200, 33, 64, seed=6)
+    d["r"] = torch.from_numpy(np.ascontiguousarray(d["r"])).pin_memory().numpy()
+    threads = lambda: len(os.listdir("/proc/self/task"))
+    with sb.Context(0) as c:
+        _host(c, _data(40, 40, 33, 64, seed=6), False)  # whatever the driver starts
+        before = threads()
+        _host(c, d, False)
+        assert threads() == before
