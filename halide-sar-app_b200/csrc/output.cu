@@ -104,16 +104,30 @@ __global__ void __launch_bounds__(256) max2_kernel(const double2 *__restrict__ i
     }
 }
 
+// Maximum over a warp of values from 0 on, whose bits order as they do.
+__device__ __forceinline__ double warp_max_bits(double v) {
+    const uint32_t hi = (uint32_t)__double2hiint(v), top = __reduce_max_sync(0xffffffffu, hi);
+    const uint32_t lo = __reduce_max_sync(0xffffffffu, hi == top ? (uint32_t)__double2loint(v) : 0u);
+    return __hiloint2double((int)top, (int)lo);
+}
+
 // max |z|^2 of the image from its partial maxima, in every thread of a CTA of 256
 __device__ __forceinline__ double image_max2(const double *__restrict__ part, int nparts) {
     double m2 = 0.0;
-    for (int i = threadIdx.x; i < nparts; i += 256) m2 = fmax(m2, part[i]);
-    for (int o = 16; o > 0; o >>= 1) m2 = fmax(m2, __shfl_xor_sync(0xffffffffu, m2, o));
+    // independent loads: one after another they are several L2 latencies ahead
+    // of the first pixel
+    for (int i0 = threadIdx.x; i0 < nparts; i0 += 8 * 256) {
+        double v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = i0 + 256 * k < nparts ? part[i0 + 256 * k] : 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) m2 = fmax(m2, v[k]);
+    }
+    m2 = warp_max_bits(m2);
     __shared__ double s[8];
     if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = m2;
     __syncthreads();
-    for (int w = 0; w < 8; ++w) m2 = fmax(m2, s[w]);
-    return m2;
+    return warp_max_bits(s[threadIdx.x & 7]);
 }
 
 // dB of one pixel.  The reference's 10 (log(|z| / m) / ln 10) takes a square

@@ -91,3 +91,27 @@ def test_db_error_is_not_above_the_f64_formulas(ctx, oracle):
     exact = 10 * np.log(a / a.max()) / np.longdouble(np.log(np.float32(10.0)))
     err = lambda d: float(np.sqrt(np.mean((d - exact) ** 2)))
     assert err(ctx.img_output_to_dB(img)) <= err(oracle.img_output_to_dB(img))
+
+
+@pytest.mark.parametrize("n", [1, 700, 5000, 300001, 3000001])
+def test_maximum_wherever_it_lies(ctx, sb, torch, n):
+    """The partial maxima of every CTA and lane count, low bits included."""
+    from sarbp_b200._lib import check, lib
+    import ctypes
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    img = torch.ones(n, 2, dtype=torch.float64, device="cuda")
+    dB = torch.empty(n, dtype=torch.float64, device="cuda")
+    u8 = torch.empty(n, dtype=torch.uint8, device="cuda")
+    for at in sorted({0, n // 7, n // 3, n // 2, max(0, n - 257), n - 1}):
+        img[at, 0] = 1.0 + 2.0 ** -40  # the high words of |z|^2 are equal
+        img[at, 1] = 1.0 + 2.0 ** -40
+        torch.cuda.synchronize()
+        check(lib().sarbp_img_output_to_dB_device(ctx.handle, p(img), n, 1, p(dB)))
+        ctx.img_output_u8_from_img_device(img.data_ptr(), n, 1, -1e-12, 0.0, u8.data_ptr())
+        ctx.synchronize()
+        assert float(dB[at]) == 0.0 and int(u8[at]) == 255
+        if n > 1:
+            rest = torch.cat([dB[:at], dB[at + 1:]])
+            assert float(rest.max()) < 0.0 and float(rest.min()) == float(rest.max())
+            assert int(torch.cat([u8[:at], u8[at + 1:]]).max()) == 0
+        img[at] = 1.0
