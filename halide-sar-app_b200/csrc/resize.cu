@@ -566,10 +566,13 @@ bool tile_shape(const ResizePlan &p, const void *in, const void *out, int *orn, 
     // 1000: 20.6 us in 4 tiles of 64 rows, 12.4 in 64 of 4; the steps 16.5)
     while (*orn > kMinTileRows && ctas() < kTileSplit) *orn = (*orn + 1) / 2;
     // A few long rows leave most of a CTA idle, and its fixed cost (3.5 us a
-    // round of 444) is more than the steps' in many rounds: 1 x 1000000 f64
-    // to 400000 is 70 us in tiles and 38 in steps, 4 x 250000 to half 31 and 43
-    const long long n = std::max(p.rows, p.orows);
-    return n > 6 || n * (long long)elem > 48 || ctas() <= 1200 * (n + 1);
+    // round of 444) is more than the steps' in many rounds, where the steps have
+    // no filter to run above all (f64, tiles and steps: 1 x 1000000 to 400000 70
+    // us and 38, 4 x 250000 to half 31 and 43; 2 x 1000000 to 3 x 1000000 64 and
+    // 48, 2 x 350000 to 3 x 350000 29 and 32, 7 x 700000 complex to 8 rows 86 and 88)
+    const long long n = std::max(p.rows, p.orows), bytes = n * (long long)elem;
+    if (p.radius[0] < 0 && p.radius[1] < 0) return n > 8 || bytes > 100 || ctas() <= (n > 1 ? 3300 : 2000);
+    return n > 6 || bytes > 48 || ctas() <= 1000 * (n + 1);
 }
 
 template <typename T, int NC>

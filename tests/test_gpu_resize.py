@@ -198,3 +198,15 @@ def test_split_tiles_round_like_the_steps(ctx, shape_in, shape_out, dtype):
     import torch
     a = np.random.default_rng(14).normal(size=shape_in + (2,)).astype(dtype)
     assert np.array_equal(_device(ctx, torch, a, shape_out), _device(ctx, torch, a, shape_out, shift=1))
+
+
+# without filters, on both sides of their line; one row has its own
+@pytest.mark.parametrize("shape_in,shape_out", [((2, 350000), (3, 350000)), ((2, 700000), (3, 700000)),
+                                                ((1, 100000), (1, 200000)), ((1, 400001), (1, 800000)),
+                                                ((7, 500000), (8, 500000))])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_long_rows_without_filters(ctx, shape_in, shape_out, dtype):
+    import torch
+    a = np.random.default_rng(15).normal(size=shape_in + (1,)).astype(dtype)
+    want = _device(ctx, torch, np.repeat(a, 3, axis=2), shape_out)[..., :1]
+    assert np.array_equal(_device(ctx, torch, a, shape_out), want)
