@@ -13,7 +13,8 @@
 namespace sarbp {
 
 // prep.cu
-void launch_prep(const DevJob *d_jobs, int njobs, cudaStream_t st);
+// longest: the most pulses or samples of a job
+void launch_prep(const DevJob *d_jobs, int njobs, int longest, cudaStream_t st);
 // One job: its descriptor goes to `job`, its work items (part-major: items
 // [0, ntiles) are part 0 of each tile, the tile list of the geometry kernels)
 // and rows [0, nrows) are listed, and counters[0 .. ncounters) cleared.

@@ -1,13 +1,14 @@
 // prep.cu -- per-job set-up kernel: Taylor windows, |k_r| filter and the
 // per-pulse geometry table, for every job of a batch in one launch.
 //
-// A cluster of kCluster CTAs per (job, part): part 0 sample window + filter
-// (+ clears the job's max|z| and status words), part 1 pulse window, part 2
-// pulse geometry.  What bounds it is the latency of the f64 cosines (a term
-// of the window each) and of the maxima over the whole window, so the
+// A cluster of up to kCluster CTAs per (job, part): part 0 sample window +
+// filter (+ clears the job's max|z| and status words), part 1 pulse window,
+// part 2 pulse geometry.  What bounds it is the latency of the f64 cosines (a
+// term of the window each) and of the maxima over the whole window, so the
 // elements are spread over the cluster's threads and the maxima go through
 // distributed shared memory: S = 8192 takes 10 us against 64 us with
-// one CTA a part, S = 1024 with P = 1999 7 us against 15 us.
+// one CTA a part, S = 1024 with P = 1999 7 us against 15 us.  In batches of many
+// jobs the start of the CTAs is the bound (see launch_prep).
 #include <cooperative_groups.h>
 
 #include "internal.h"
@@ -22,8 +23,8 @@ constexpr int kKeep = 4;  // window values a thread keeps between the maximum an
 
 namespace cg = cooperative_groups;
 
-// Maxima of N values over the cluster (fmax: the order does not change them).
-template <int N>
+// Maxima of N values over a cluster of CL CTAs (fmax: the order does not change them).
+template <int CL, int N>
 __device__ void cluster_max(double (&v)[N]) {
     __shared__ double part[kPrepThreads / 32][N], mine[N];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -37,14 +38,19 @@ __device__ void cluster_max(double (&v)[N]) {
         for (int w = 1; w < kPrepThreads / 32; ++w) m = fmax(m, part[w][threadIdx.x]);
         mine[threadIdx.x] = m;
     }
-    cg::cluster_group cl = cg::this_cluster();
-    cl.sync();
-    for (int k = 0; k < N; ++k) {
-        double m = mine[k];
-        for (int r = 0; r < kCluster; ++r) m = fmax(m, cl.map_shared_rank(mine, r)[k]);
-        v[k] = m;
+    if constexpr (CL == 1) {
+        __syncthreads();
+        for (int k = 0; k < N; ++k) v[k] = mine[k];
+    } else {
+        cg::cluster_group cl = cg::this_cluster();
+        cl.sync();
+        for (int k = 0; k < N; ++k) {
+            double m = mine[k];
+            for (int r = 0; r < CL; ++r) m = fmax(m, cl.map_shared_rank(mine, r)[k]);
+            v[k] = m;
+        }
+        cl.sync();  // no CTA leaves while another reads its maxima
     }
-    cl.sync();  // no CTA leaves while another reads its maxima
 }
 
 // Taylor window before normalisation, signal.h:43-45:
@@ -88,9 +94,10 @@ __device__ void image_frame(const DevJob &jb, double (&E)[3][3]) {
     E[1][2] = 0.0;
 }
 
+template <int CL>
 __device__ __forceinline__ void prep_part(const DevJob &jb, int what, int rank) {
     const int first = rank * kPrepThreads + threadIdx.x;  // this thread's first element
-    constexpr int kStride = kCluster * kPrepThreads;
+    constexpr int kStride = CL * kPrepThreads;
     if (what == 0 || what == 1) {
         const int num = what == 0 ? jb.S : jb.P;
         float *dst = what == 0 ? jb.wS : jb.wP;
@@ -102,7 +109,7 @@ __device__ __forceinline__ void prep_part(const DevJob &jb, int what, int rank) 
             m[0] = fmax(m[0], keep[i]);
         }
         for (int x = first + kKeep * kStride; x < num; x += kStride) m[0] = fmax(m[0], taylor_w(jb, num, x));
-        cluster_max(m);
+        cluster_max<CL>(m);
 #pragma unroll
         for (int i = 0; i < kKeep; ++i) {
             const int x = first + i * kStride;
@@ -166,7 +173,7 @@ __device__ __forceinline__ void prep_part(const DevJob &jb, int what, int rank) 
                 la[3] = 0.0;  // no bound from this job's positions
             }
         }
-        cluster_max(la);
+        cluster_max<CL>(la);
         if (first == 0) {
             for (int i = 0; i < 3; ++i) {
                 jb.sc->los_abs[i] = la[i];
@@ -177,9 +184,13 @@ __device__ __forceinline__ void prep_part(const DevJob &jb, int what, int rank) 
     }
 }
 
-__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
-    prep_kernel(const DevJob *__restrict__ jobs) {
-    prep_part(jobs[blockIdx.x / kCluster], blockIdx.y, blockIdx.x % kCluster);
+template <int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPrepThreads)
+    prep_cluster_kernel(const DevJob *__restrict__ jobs) {
+    prep_part<CL>(jobs[blockIdx.x / CL], blockIdx.y, blockIdx.x % CL);
+}
+__global__ void __launch_bounds__(kPrepThreads) prep_kernel(const DevJob *__restrict__ jobs) {
+    prep_part<1>(jobs[blockIdx.x], blockIdx.y, 0);
 }
 
 // The same for one job whose descriptor comes as a kernel parameter, which
@@ -195,13 +206,26 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kPrepThreads)
     for (int i = i0; i < l.nitems; i += kAll) l.items[i] = WorkItem{0, i % l.ntiles, i / l.ntiles};
     for (int i = i0; i < l.nrows; i += kAll) l.rows[i] = RowItem{0, i};
     for (int i = i0; i < l.ncounters; i += kAll) l.counters[i] = 0;
-    prep_part(job, blockIdx.y, blockIdx.x);
+    prep_part<kCluster>(job, blockIdx.y, blockIdx.x);
 }
 
 }  // namespace
 
-void launch_prep(const DevJob *d_jobs, int njobs, cudaStream_t st) {
-    prep_kernel<<<dim3(njobs * kCluster, 3), kPrepThreads, 0, st>>>(d_jobs);
+// A thread's turn of an element takes about 1.4 us and the start of a CTA of a
+// cluster 7 ns of the launch, so of clusters of C CTAs the best C is about the
+// root of longest / (4 njobs); each line lies half-way to the next size.  300 jobs of
+// 60 x 64: 16 us with one CTA a part, 69 with eight; 96 of 1999 x 1024: 20 with
+// two, 37 and 23 with eight and one; 48 of 200 x 8192: 27 with eight, 66 with one.
+void launch_prep(const DevJob *d_jobs, int njobs, int longest, cudaStream_t st) {
+    auto pays = [&](int c) { return longest > kPrepThreads * c / 2 && 2ll * c * c * njobs <= longest; };
+    if (pays(8))
+        prep_cluster_kernel<8><<<dim3(njobs * 8, 3), kPrepThreads, 0, st>>>(d_jobs);
+    else if (pays(4))
+        prep_cluster_kernel<4><<<dim3(njobs * 4, 3), kPrepThreads, 0, st>>>(d_jobs);
+    else if (pays(2))
+        prep_cluster_kernel<2><<<dim3(njobs * 2, 3), kPrepThreads, 0, st>>>(d_jobs);
+    else
+        prep_kernel<<<dim3(njobs, 3), kPrepThreads, 0, st>>>(d_jobs);
 }
 
 cudaError_t launch_prep_single(const DevJob &job, const SingleLists &lists, cudaStream_t st) {

@@ -628,7 +628,9 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
                                                 (int)nrows_total, d_cnt, (int)(cnt_bytes / sizeof(int))}, st);
         if (e != cudaSuccess) return cuda_fail(e, "set-up launch");
     } else {
-        launch_prep(d_jobs, njobs, st);
+        int longest = 0;
+        for (int i = 0; i < njobs; ++i) longest = std::max({longest, jobs[i].npulses, jobs[i].nsamples});
+        launch_prep(d_jobs, njobs, longest, st);
     }
     dev_->launches++;
     if ((e = rec(1)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");

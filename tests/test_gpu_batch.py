@@ -158,3 +158,29 @@ def test_taylor_above_30_db_float_window_matches_oracle(ctx, sb, oracle):
         ctx.run_jobs([ref_job])
     assert e.value.code == sb.ERR_INVALID and b"30 dB" in str(e.value).encode()
     ref_job.taylor_mode = sb.TAYLOR_FLOAT
+
+
+# the set-up's clusters of 8, 4, 2 and 1 CTAs, on both sides of each line (one
+# job alone: 8); windows, filter and pulse table are the same whichever it is
+@pytest.mark.parametrize("P,S", [(1100, 70), (40, 1100)])
+def test_many_jobs_are_set_up_as_one(ctx, sb, P, S):
+    import torch
+    from sarbp_b200 import synth
+    dev = lambda a, t: torch.from_numpy(np.ascontiguousarray(a, t)).cuda()  # noqa: E731
+    d = synth.make("plain_small", seed=21, with_r=True, overrides=dict(P=P, S=S, n=32, extent=6.4, taylor=25))
+    t = [dev(d["phs"].view(np.float32), np.float32), dev(d["k_r"], np.float32), dev(d["pos"], np.float32),
+         dev(d["r"], np.float64)]
+    out = torch.zeros(140, 32, 32, 2, dtype=torch.float64, device="cuda")
+    job = lambda o: sb.make_job(S, P, d["N_fft"], 25, 32, 32, d["delta_r"], t[0].data_ptr(), t[1].data_ptr(),  # noqa: E731
+                                t[2].data_ptr(), o.data_ptr(), r=t[3].data_ptr(), precision=sb.PREC_COMPAT)
+    torch.cuda.synchronize()
+    ctx.run_jobs([job(out[0])])
+    ctx.synchronize()
+    want = out[0].clone()
+    assert float(want.abs().max()) > 0
+    for m in (2, 8, 9, 34, 35, 137, 138):
+        out.zero_()
+        torch.cuda.synchronize()
+        ctx.run_jobs([job(out[i]) for i in range(m)])
+        ctx.synchronize()
+        assert torch.equal(out[:m], want.expand(m, -1, -1, -1)), m
