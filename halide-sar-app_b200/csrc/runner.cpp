@@ -581,9 +581,6 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         dj.sum_parts = sum_parts;
         dj.parts = nsplit[i] > 1 ? reinterpret_cast<float2 *>(sbase + lay[i].parts) : nullptr;
     }
-    // The caller's inputs may still be on their way on the slabs' copy stream
-    // (and the descriptors of a batch go up behind them)
-    cudaStream_t ms = (slabs && slabs->copy_stream) ? slabs->copy_stream : st;
     if (!single) {
         RowItem *hr = reinterpret_cast<RowItem *>(h + o_rows);
         for (const RowGroup &g : row_groups)
@@ -591,12 +588,16 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         std::memcpy(h + o_items, items.data(), items.size() * sizeof(WorkItem));
         std::memcpy(h + o_tiles, tiles.data(), tiles.size() * sizeof(WorkItem));
         std::memcpy(h + o_comb, combine.data(), combine.size() * sizeof(int));
-        e = cudaMemcpyAsync(d, h, meta_bytes, cudaMemcpyHostToDevice, ms);
+        e = cudaMemcpyAsync(d, h, meta_bytes, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess && !for_graph) e = cudaEventRecord(meta_done_, st);
         if (e != cudaSuccess) return cuda_fail(e, "copying descriptors");
+    } else if (slabs && slabs->copy_stream && slabs->copy_stream != st) {
+        // the caller's inputs may still be on their way
+        // (not meta_done_: an earlier batch's descriptors may still be read)
+        e = cudaEventRecord(front_done_, slabs->copy_stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(st, front_done_, 0);
+        if (e != cudaSuccess) return cuda_fail(e, "ordering the input copies");
     }
-    if (!for_graph && (!single || ms != st)) e = cudaEventRecord(meta_done_, ms);
-    if (e == cudaSuccess && ms != st) e = cudaStreamWaitEvent(st, meta_done_, 0);
-    if (e != cudaSuccess) return cuda_fail(e, "ordering the descriptor copy");
 
     DevJob *d_jobs = reinterpret_cast<DevJob *>(d + o_jobs);
     RowItem *d_rows = reinterpret_cast<RowItem *>(d + o_rows);

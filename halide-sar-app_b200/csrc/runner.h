@@ -84,17 +84,13 @@ struct SlabSpec {
     cudaStream_t aux = nullptr;
     const cudaEvent_t *ready = nullptr;  // [nslabs] or NULL
     const cudaEvent_t *done = nullptr;   // [nslabs]
-    // Called once the descriptors and the range compression are enqueued and
-    // before any slab waits on `ready`: the place to issue the slabs' input
-    // copies and record `ready`.  Host-to-device copies of all streams share
-    // the copy engine in issue order, so copies issued earlier would hold
-    // back the batch's own descriptor upload.
+    // Called once the set-up and the range compression are enqueued and before
+    // any slab waits on `ready`: the place to issue the slabs' input copies and
+    // record `ready`.  Copies of pageable memory hold the calling thread, so
+    // issued earlier they would delay those launches.
     std::function<cudaError_t()> before_slabs;
-    // When set, the batch's descriptors are uploaded on this stream (where
-    // the caller has already queued the phase-history copies) and the
-    // kernels wait for them there: the copy engine runs one stream's queue
-    // ahead of another's, so a descriptor copy on the compute stream could
-    // wait behind every queued input copy.
+    // When set, the stream on which the caller has queued the copies of the
+    // inputs other than the pixel positions: the set-up waits for them.
     cudaStream_t copy_stream = nullptr;
 };
 
@@ -104,12 +100,13 @@ public:
     ~Runner();
     // Validates and enqueues jobs on st.  Returns SARBP_OK or an error code
     // (no device work is enqueued on a validation error).
-    // With q_out set, only range compression runs and job 0's profiles are
-    // copied there.
+    // With q_out set, only range compression runs and job 0's profiles go
+    // there: stored by its kernels where they can write q_out, else copied.
     // With for_graph set the call is being captured into a CUDA graph: no
-    // stage events, no wait on the previous descriptor copy (the captured
-    // copy re-reads this Runner's pinned descriptors at every replay, so the
-    // Runner must not enqueue anything else afterwards), and every buffer
+    // stage events, no wait on the previous descriptor copy (for several jobs
+    // the captured copy re-reads this Runner's pinned descriptors at every
+    // replay, and the kernels use its device memory, so the Runner must not
+    // enqueue anything else afterwards), and every buffer
     // must already be large enough (an uncaptured enqueue of the same jobs
     // comes first).
     // With resident_qp, job i whose resident_qp[i] is non-NULL uses those
@@ -142,7 +139,7 @@ private:
     DeviceBuffer scratch_, meta_;
     PinnedBuffer host_meta_;
     cudaEvent_t meta_done_ = nullptr;  // host_meta_ may be rewritten after this
-    cudaEvent_t front_done_ = nullptr; // range compression done (slabbed runs)
+    cudaEvent_t front_done_ = nullptr; // slabbed runs: inputs copied, then range compression done
     // Tile geometry and range compression run beside each other, one of them on
     // side_ or side_high_ (high priority); fork_/join_ order them.
     cudaStream_t side_ = nullptr, side_high_ = nullptr;
