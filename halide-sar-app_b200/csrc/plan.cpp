@@ -4,10 +4,12 @@
 // enqueued once for real, which sizes every scratch buffer and builds the
 // twiddle tables, and then captured into a CUDA graph: prep, one range
 // compression launch per FFT length, tile geometry, the persistent
-// backprojection over the (job, tile, pulse part) work list and the u8 stage.  Each
-// replay re-reads the job descriptors from the plan's own pinned copy, so the
-// input arrays may hold new data between replays but must keep their
-// addresses and shapes.
+// backprojection over the (job, tile, pulse part) work list, the combine
+// kernel where jobs formed in parts need it, and the u8 stage.  A replay of
+// several jobs copies their descriptors from the plan's own pinned memory; one
+// job's is a parameter of the captured set-up kernel.  Either way the input
+// arrays may hold new data between replays but must keep their addresses and
+// shapes.
 //
 // The autotuner times the whole batch (set-up through backprojection) over
 // a set of pixel-tile shapes, CTAs per SM and pulse-chunk depths, keeps the
