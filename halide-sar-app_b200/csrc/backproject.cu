@@ -421,9 +421,17 @@ __device__ __forceinline__ bool stage_windows(const DevJob &jb, int lane, int p0
         }
         const int lo = max(base, 0), hi = min(base + W, N);
         if (hi > lo) bulk_copy(dst + (lo - base), row + lo, (uint32_t)(hi - lo) * 16u, &sm.mbar_win[b]);
-        // bins < 0 read Q[0] twice, bins >= N-1 read Q[N-1] twice (clamp)
-        for (int j = 0; j < W && base + j < 0; ++j) dst[j] = row[N];
-        for (int j = max(N - base, 0); j < W; ++j) dst[j] = row[N - 1];
+        // bins < 0 read Q[0] twice, bins >= N-1 read Q[N-1] twice (clamp); one
+        // load each: with a load an entry, tiles off the range swath waited for
+        // this loop (1612x1985 x 841, most of it off the swath: 5880 us, 4044 so)
+        if (base < 0) {
+            const float4 q = row[N];
+            for (int j = min(W, -base) - 1; j >= 0; --j) dst[j] = q;
+        }
+        if (base + W > N) {
+            const float4 q = row[N - 1];
+            for (int j = max(N - base, 0); j < W; ++j) dst[j] = q;
+        }
     }
     ok = mbar_wait(&sm.mbar_win[b], uses[2 + b] & 1u) && ok;
     uses[2 + b]++;

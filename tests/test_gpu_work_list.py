@@ -89,3 +89,18 @@ def test_parts_summed_by_the_last_item(ctx, torch, parts, P):
         a.out.fill_(-7.0)
         again = a.run(ctx, jobs=[a.job, b.job], pulse_parts=parts)
         assert np.array_equal(first[0], again[0]) and np.array_equal(first[1], again[1])
+
+
+# range windows wholly or partly below and above the profile: the clamped edge
+# pairs; narrow and wide windows
+@pytest.mark.parametrize("upsample,pixel", [(2, 0.8), (6, 1.6), (1, 2.5)])
+def test_tiles_off_the_range_swath(ctx, oracle, torch, upsample, pixel):
+    nu, nv, P = 230, 190, 70
+    d = synth.make_from(_cfg(P, 3, S=64, upsample=upsample))
+    u, v = (np.arange(nu) - nu // 2) * pixel, (np.arange(nv) - nv // 2) * pixel
+    r = sb.pixel_locs(u, v, d["u_hat"], d["v_hat"])
+    got = ctx.backprojection_cuda(d["phs"], d["k_r"], 20, d["N_fft"], d["delta_r"], u, v, d["pos"], r)
+    idx = np.random.default_rng(1).choice(nu * nv, 4000, replace=False)
+    want = oracle.backprojection(d["phs"], d["k_r"], 20, d["N_fft"], d["delta_r"], d["pos"], r, nu, nv,
+                                 mode=oracle.MODE_FP64, out_idx=idx)
+    assert np.linalg.norm(got.reshape(-1)[idx] - want) < 1e-4 * np.linalg.norm(want)
