@@ -45,12 +45,13 @@
 // A job with too few tiles to fill the resident CTAs has each
 // tile split into nsplit items over consecutive pulse ranges; each stores
 // its sums into its own slice of the job's parts buffer.  Where every CTA has
-// one item, the CTA that completes a tile's last part (a counter per tile) adds
-// the slices in part order, so that the image does not depend on which CTA that
-// is (256^2 x 300: 6 us less than a launch that does so).  In longer lists
-// the fences would hold back each item (4 jobs of 128^2 and 256^2 pixels in 688
-// items: 98 us against 72 and 6 for the combine kernel), and the combine
-// kernel adds the slices in the same order.
+// one item and a tile at most kMaxSumParts, the CTA that completes a tile's last
+// part (a counter per tile) adds the slices in part order, so that the image
+// does not depend on which CTA that is (256^2 x 300: 6 us less than a launch
+// that does so).  With more parts its loads, one part after another, take longer
+// than that launch, and in longer lists the fences would hold back each item (4
+// jobs of 128^2 and 256^2 pixels in 688 items: 98 us against 72 and 6 for the
+// combine kernel); there the combine kernel adds the slices in the same order.
 //
 // Naive kernel: the same quantity with plain FP32 range |pos| - |r - pos|
 // and phase k_c * dr per pixel*pulse; kept as the precision-study baseline.

@@ -74,6 +74,11 @@ cudaError_t init_backproject_attributes();
 // d_counter: kBpCounterBytes of device memory (kBpDealBytes with kDealPulses),
 // zero before a persistent launch; word kBpZeroWord stays zero
 constexpr int kBpZeroWord = 3;
+// Most pulse parts that a tile's last item adds itself: it reads them one after
+// another, the combine kernel several at once (20 tiles of 118x147 pixels in
+// 16 parts replayed: 83 us a plan in place, 64 with the combine kernel; in
+// four parts they are equal)
+constexpr int kMaxSumParts = 4;
 constexpr int kBpCounterBytes = 256, kBpDealSms = 252, kBpDealBytes = 16 + 4 * kBpDealSms;
 cudaError_t launch_backproject(const BpLaunch &L, const DevJob *d_jobs, const WorkItem *d_items,
                                int nitems, int *d_counter, cudaStream_t st);

@@ -242,10 +242,9 @@ extern "C" int sarbp_backprojection_noalloc(const sarbp_job *job, void *cuda_str
     L.grid = (int)std::min<long long>((long long)occ * num_sms, (long long)nitems);
     L.deal.how = kDealItems;  // one job: its parts differ by a pulse at most
     dj.nsplit = nsplit;
-    // a tile's parts are added by its last item where every CTA has one item, by
-    // the combine kernel in longer lists (400^2 x 900: 176 us a call in place,
-    // 154 so)
-    dj.sum_parts = nitems <= (size_t)L.grid;
+    // a tile's few parts are added by its last item where every CTA has one item,
+    // else by the combine kernel (400^2 x 900: 176 us a call in place, 154 so)
+    dj.sum_parts = nsplit <= kMaxSumParts && nitems <= (size_t)L.grid;
     dj.parts = nsplit > 1 ? reinterpret_cast<float2 *>(sb + o_parts) : nullptr;
 
     DevJob *d_job = reinterpret_cast<DevJob *>(sb + o_job);

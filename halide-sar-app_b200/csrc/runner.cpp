@@ -518,13 +518,14 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         nrows_total += kv.second.size();
     }
 
-    // a tile's parts are added by its last item where every CTA has one item
+    // a tile's few parts are added by its last item where every CTA has one item
     const int resident_bp = any_split ? bp_max_active_blocks(L) * dev_->num_sms : 0;
-    const bool sum_parts = any_split && L.persistent && nitems <= (size_t)resident_bp;
+    const bool one_round = any_split && L.persistent && nitems <= (size_t)resident_bp;
+    auto sum_parts = [&](int i) { return one_round && nsplit[i] <= kMaxSumParts; };
     std::vector<int> combine;  // jobs that need the combine kernel
     long long combine_px = 0;
     for (int i = 0; i < njobs; ++i)
-        if (nsplit[i] > 1 && !sum_parts) {
+        if (nsplit[i] > 1 && !sum_parts(i)) {
             combine.push_back(i);
             combine_px = std::max(combine_px, (long long)jobs[i].nu * jobs[i].nv);
         }
@@ -578,7 +579,7 @@ int Runner::enqueue(const sarbp_job *jobs, int njobs, const sarbp_opts *opts, cu
         dj.u8_chunk0 = u8_total;
         if (j.out_u8) u8_total += u8_chunks((long long)j.nu * j.nv);
         dj.nsplit = nsplit[i];
-        dj.sum_parts = sum_parts;
+        dj.sum_parts = sum_parts(i);
         dj.parts = nsplit[i] > 1 ? reinterpret_cast<float2 *>(sbase + lay[i].parts) : nullptr;
     }
     if (!single) {

@@ -183,9 +183,9 @@ int sarbp_range_compress_device(sarbp_ctx *ctx, const sarbp_job *job,
  * compression launch per distinct N_fft, and one persistent backprojection
  * launch over a (job, pixel tile, pulse part) work list ordered
  * longest-first (small jobs split their tiles' pulses into parts, see
- * sarbp_opts.pulse_parts), then, where the list is longer than the resident
- * CTAs, one combine launch for the jobs formed in parts.  Enqueued on the
- * context's stream, not synchronised.
+ * sarbp_opts.pulse_parts), then one combine launch for the jobs formed in
+ * more than a few parts, or in parts in a list longer than the resident CTAs.
+ * Enqueued on the context's stream, not synchronised.
  */
 int sarbp_batch_device(sarbp_ctx *ctx, const sarbp_job *jobs, int njobs,
                        const sarbp_opts *opts);

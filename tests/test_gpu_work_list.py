@@ -104,3 +104,16 @@ def test_tiles_off_the_range_swath(ctx, oracle, torch, upsample, pixel):
     want = oracle.backprojection(d["phs"], d["k_r"], 20, d["N_fft"], d["delta_r"], d["pos"], r, nu, nv,
                                  mode=oracle.MODE_FP64, out_idx=idx)
     assert np.linalg.norm(got.reshape(-1)[idx] - want) < 1e-4 * np.linalg.norm(want)
+
+
+def test_parts_summed_in_place_beside_parts_combined(ctx, torch):
+    """One round of items: a job in two parts (added by a tile's last item)
+    and one in many (the combine kernel), as alone."""
+    a, b = _Job(torch, 300, 300, 90, seed=31), _Job(torch, 70, 60, 620, seed=32)
+    alone = [a.run(ctx), b.run(ctx)]
+    for _ in range(3):
+        a.out.fill_(-7.0)
+        b.out.fill_(-7.0)
+        a.run(ctx, jobs=[a.job, b.job])
+        for j, (img, u8) in zip((a, b), alone):
+            assert np.array_equal(img, j.out.cpu().numpy()) and np.array_equal(u8, j.u8.cpu().numpy())
