@@ -182,25 +182,33 @@ cudaError_t HostStager::settle(Slot &s, int i) {
     return cudaSuccess;
 }
 
-// The slots; false where there is no page-locked memory to be had.  A
+// The slots; false where there is no page-locked memory to be had (and in a
+// forked child, which has no mapping of them).  A
 // context's first call waits for the locking of 16 MB, so they are mapped in
 // huge pages where the system has them and the threads touch the pages ahead
 // of it: 1.2 ms, against 2.9 without the threads and 8 with cudaMallocHost
 // (the first 768^2 x 800 call of a context 6 ms, as with the driver's own
 // staging, against 8 and 20).
 bool HostStager::ready() {
-    if (pin_) return true;
+    if (pin_) return pid_ == getpid();
     constexpr size_t kHuge = 2 << 20, kBytes = kSlotBytes * kSlots;
     void *p = mmap(nullptr, kBytes + kHuge, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
     if (p == MAP_FAILED) return false;
     char *at = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(p) + kHuge - 1) / kHuge * kHuge);
     madvise(at, kBytes, MADV_HUGEPAGE);
+    // A fork would make the pages copies-on-write: the caller's next write to a
+    // slot could go to a new page, the device's transfer to the old one.
+    if (madvise(at, kBytes, MADV_DONTFORK) != 0) {
+        munmap(p, kBytes + kHuge);
+        return false;
+    }
     threads_.zero(at, kBytes, kHuge);  // a page a thread, ahead of the locking
     if (cudaHostRegister(at, kBytes, cudaHostRegisterPortable) != cudaSuccess) {
         cudaGetLastError();
         munmap(p, kBytes + kHuge);
         return false;
     }
+    pid_ = getpid();
     map_ = p;
     map_bytes_ = kBytes + kHuge;
     pin_ = at;
@@ -277,7 +285,7 @@ void HostStager::release() {
         if (s.ev) cudaEventDestroy(s.ev);
         s = Slot{};
     }
-    if (pin_) {
+    if (pin_ && pid_ == getpid()) {  // (a child may have other things mapped there)
         cudaHostUnregister(pin_);
         munmap(map_, map_bytes_);
     }

@@ -83,6 +83,7 @@ private:
     void abandon();  // drops downloads that a failed call left behind
     CopyThreads threads_;
     char *pin_ = nullptr;
+    pid_t pid_ = 0;        // the process that locked the slots
     void *map_ = nullptr;  // the mapping that holds pin_
     size_t map_bytes_ = 0;
     Slot slots_[kSlots];

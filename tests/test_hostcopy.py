@@ -59,6 +59,18 @@ static double cpu_seconds() {
     getrusage(RUSAGE_SELF, &r);
     return r.ru_utime.tv_sec + r.ru_stime.tv_sec + 1e-6 * (r.ru_utime.tv_usec + r.ru_stime.tv_usec);
 }
+// kB of mappings that a forked child does not get
+static long kept_from_children() {
+    FILE *f = fopen("/proc/self/smaps", "r");
+    char line[4096];
+    long size = 0, total = 0;
+    while (fgets(line, sizeof(line), f)) {
+        sscanf(line, "Size: %ld kB", &size);
+        if (!strncmp(line, "VmFlags:", 8) && strstr(line, " dc")) total += size;
+    }
+    fclose(f);
+    return total;
+}
 // n bytes up and down again; whether they arrived
 static bool round_trip(HostStager &s, size_t n, unsigned seed) {
     std::vector<char> a(n), dev(n), b(n);
@@ -106,6 +118,9 @@ int main(int, char **argv) {
             return 1;
         }
         ok = ok && WIFEXITED(st) && WEXITSTATUS(st) == 0 && round_trip(*s, 9000001, 3);
+    } else if (!strcmp(argv[1], "slots_stay_out_of_a_child")) {
+        ok = round_trip(*s, 9000001, 6);
+        ok = ok && kept_from_children() >= (16 << 10);
     } else if (!strcmp(argv[1], "no_page_locked_memory")) {
         g_no_pin = true;
         ok = round_trip(*s, 9000001, 4);
@@ -133,10 +148,13 @@ def exe(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("what", ["data", "fork", "nothing_staged", "idle", "no_page_locked_memory"])
+@pytest.mark.parametrize("what", ["data", "fork", "nothing_staged", "idle", "no_page_locked_memory",
+                                  "slots_stay_out_of_a_child"])
 def test_staged_copies(exe, what):
     """The bytes arrive; a forked child copies by itself and may drop the
     object; threads start with the first staged copy and sleep while nothing is
-    copied; without page-locked memory the copies are the driver's."""
+    copied; without page-locked memory the copies are the driver's; a fork does
+    not make the slots' pages copies-on-write, under which the device would
+    go on with the old pages."""
     p = subprocess.run([exe, what], capture_output=True, text=True, timeout=120)
     assert p.returncode == 0 and p.stdout.strip() == "ok", p.stdout
